@@ -18,16 +18,38 @@ __device__ __forceinline__ T sp64_t(T x) { return mlog(1.0 + mexp(x)) + 1e-6; }
 
 // The model formulas on a scalar type T: double (eval_model_f64 and
 // model_grad_f64 below) or the forward-mode Dual of dual64.cuh (the Laplace
-// Hessian).
+// Hessian).  E gives what depends on the parameters alone, e(k) = exp(p[k])
+// of the logarithmic ones (log_param) and Arnett's nickel fraction e(3):
+// formed where the formula needs it (ExpNow), or once per parameter vector by
+// callers that evaluate it at many times (ExpTable).
+__host__ __device__ constexpr bool log_param(int m, int k) {
+    return k == 0 || (m == 0 && (k == 3 || k == 4)) || (m == 1 && (k == 2 || k == 4 || k == 5)) ||
+           (m == 2 && (k == 3 || k == 4)) || (m == 3 && k == 2) || (m == 4 && (k == 2 || k == 3)) ||
+           (m == 5 && k == 3) || (m == 6 && k == 2);
+}
 template <class T>
-__device__ inline T eval_model_t(int m, const T* p, T t) {
+__device__ __forceinline__ T nickel_fraction(T p3) { return 1.0 / (1.0 + mexp(-p3)); }
+template <class T>
+struct ExpNow {
+    int m;
+    const T* p;
+    __device__ __forceinline__ T operator()(int k) const {
+        return m == 3 && k == 3 ? nickel_fraction(p[3]) : mexp(p[k]);
+    }
+};
+struct ExpTable {
+    const double* e;
+    __device__ __forceinline__ double operator()(int k) const { return e[k]; }
+};
+template <class T, class E>
+__device__ __forceinline__ T eval_model_e(int m, const T* p, const E& e, T t) {
     switch (m) {
         case 0: {
-            T a = mexp(p[0]), b = p[1], dt = t - p[2], tr = mexp(p[3]), tf = mexp(p[4]);
+            T a = e(0), b = p[1], dt = t - p[2], tr = e(3), tf = e(4);
             return a * mexp(-dt / tf) * (1.0 / (1.0 + mexp(-dt / tr))) + b;
         }
         case 1: {
-            T a = mexp(p[0]), beta = p[1], gamma = mexp(p[2]), ph = t - p[3], tr = mexp(p[4]), tf = mexp(p[5]);
+            T a = e(0), beta = p[1], gamma = e(2), ph = t - p[3], tr = e(4), tf = e(5);
             T sig = 1.0 / (1.0 + mexp(-ph / tr));
             T w = 1.0 / (1.0 + mexp(-10.0 * (ph - gamma)));
             T pl = 1.0 - beta * ph;
@@ -35,35 +57,35 @@ __device__ inline T eval_model_t(int m, const T* p, T t) {
             return a * sig * ((1.0 - w) * pl + w * pr);
         }
         case 2: {
-            T a = mexp(p[0]), b = p[1], ph = t - p[2], tr = mexp(p[3]), tf = mexp(p[4]), al = p[5];
+            T a = e(0), b = p[1], ph = t - p[2], tr = e(3), tf = e(4), al = p[5];
             T sig = 1.0 / (1.0 + mexp(-ph / tr));
             T w = 1.0 + sp64_t(ph) / tf;
             return a * sig * mpow(w, -al) + b;
         }
         case 3: {
-            T a = mexp(p[0]), ph = t - p[1], tm = mexp(p[2]);
+            T a = e(0), ph = t - p[1], tm = e(2);
             T ps = sp64_t(ph);
-            T f = 1.0 / (1.0 + mexp(-p[3]));
+            T f = e(3);
             T heat = f * mexp(-ps / 8.8) + (1.0 - f) * mexp(-ps / 111.3);
             T x = ps / tm;
             return a * heat * (1.0 - mexp(-x * x));
         }
         case 4: {
-            T a = mexp(p[0]), ph = t - p[1], tsd = mexp(p[2]), td = mexp(p[3]);
+            T a = e(0), ph = t - p[1], tsd = e(2), td = e(3);
             T ps = sp64_t(ph);
             T w = 1.0 + ps / tsd;
             T x = ps / td;
             return a * (1.0 / (w * w)) * (1.0 - mexp(-x * x));
         }
         case 5: {
-            T a = mexp(p[0]), ph = t - p[1], n = p[2], ttr = mexp(p[3]);
+            T a = e(0), ph = t - p[1], n = p[2], ttr = e(3);
             T sig5 = 1.0 / (1.0 + mexp(-ph * 5.0));
             T ps = sp64_t(ph);
             T r = ps / ttr;
             return a * sig5 * mpow(ps, -n) * mexp(-r * r);
         }
         default: {
-            T a = mexp(p[0]), ph = t - p[1], tb = mexp(p[2]), a1 = p[3], a2 = p[4];
+            T a = e(0), ph = t - p[1], tb = e(2), a1 = p[3], a2 = p[4];
             T ps = sp64_t(ph);
             T lr = mlog(ps / tb);
             T u = mexp(2.0 * a1 * lr) + mexp(2.0 * a2 * lr);
@@ -71,15 +93,19 @@ __device__ inline T eval_model_t(int m, const T* p, T t) {
         }
     }
 }
+template <class T>
+__device__ inline T eval_model_t(int m, const T* p, T t) {
+    return eval_model_e(m, p, ExpNow<T>{m, p}, t);
+}
 __device__ inline double eval_model_f64(int m, const double* p, double t) { return eval_model_t<double>(m, p, t); }
 
 // Analytic d flux / d theta (src/parametric.rs:213-509); the sigma_extra
 // slot is 0.
-template <class T>
-__device__ inline void model_grad_t(int m, const T* p, T t, T* o) {
+template <class T, class E>
+__device__ __forceinline__ void model_grad_e(int m, const T* p, const E& e, T t, T* o) {
     switch (m) {
         case 0: {
-            T a = mexp(p[0]), dt = t - p[2], tr = mexp(p[3]), tf = mexp(p[4]);
+            T a = e(0), dt = t - p[2], tr = e(3), tf = e(4);
             T sig = 1.0 / (1.0 + mexp(-dt / tr));
             T base = a * mexp(-dt / tf) * sig;
             o[0] = base; o[1] = T(1.0);
@@ -90,7 +116,7 @@ __device__ inline void model_grad_t(int m, const T* p, T t, T* o) {
             return;
         }
         case 1: {
-            T a = mexp(p[0]), beta = p[1], gamma = mexp(p[2]), ph = t - p[3], tr = mexp(p[4]), tf = mexp(p[5]);
+            T a = e(0), beta = p[1], gamma = e(2), ph = t - p[3], tr = e(4), tf = e(5);
             const double k = 10.0;
             T sig = 1.0 / (1.0 + mexp(-ph / tr));
             T w = 1.0 / (1.0 + mexp(-k * (ph - gamma)));
@@ -113,7 +139,7 @@ __device__ inline void model_grad_t(int m, const T* p, T t, T* o) {
             return;
         }
         case 2: {
-            T a = mexp(p[0]), ph = t - p[2], tr = mexp(p[3]), tf = mexp(p[4]), al = p[5];
+            T a = e(0), ph = t - p[2], tr = e(3), tf = e(4), al = p[5];
             T sig = 1.0 / (1.0 + mexp(-ph / tr));
             T ps = sp64_t(ph);
             T sp = mexp(ph) / (1.0 + mexp(ph));
@@ -130,10 +156,10 @@ __device__ inline void model_grad_t(int m, const T* p, T t, T* o) {
             return;
         }
         case 3: {
-            T a = mexp(p[0]), ph = t - p[1], tm = mexp(p[2]);
+            T a = e(0), ph = t - p[1], tm = e(2);
             T ps = sp64_t(ph);
             T sp = mexp(ph) / (1.0 + mexp(ph));
-            T f = 1.0 / (1.0 + mexp(-p[3]));
+            T f = e(3);
             T eni = mexp(-ps / 8.8), eco = mexp(-ps / 111.3);
             T heat = f * eni + (1.0 - f) * eco;
             T x = ps / tm;
@@ -149,7 +175,7 @@ __device__ inline void model_grad_t(int m, const T* p, T t, T* o) {
             return;
         }
         case 4: {
-            T a = mexp(p[0]), ph = t - p[1], tsd = mexp(p[2]), td = mexp(p[3]);
+            T a = e(0), ph = t - p[1], tsd = e(2), td = e(3);
             T ps = sp64_t(ph);
             T sp = mexp(ph) / (1.0 + mexp(ph));
             T w = 1.0 + ps / tsd;
@@ -166,7 +192,7 @@ __device__ inline void model_grad_t(int m, const T* p, T t, T* o) {
             return;
         }
         case 5: {
-            T a = mexp(p[0]), ph = t - p[1], n = p[2], ttr = mexp(p[3]);
+            T a = e(0), ph = t - p[1], n = p[2], ttr = e(3);
             T sig5 = 1.0 / (1.0 + mexp(-ph * 5.0));
             T ps = sp64_t(ph);
             T sp = mexp(ph) / (1.0 + mexp(ph));
@@ -183,7 +209,7 @@ __device__ inline void model_grad_t(int m, const T* p, T t, T* o) {
             return;
         }
         default: {
-            T a = mexp(p[0]), ph = t - p[1], tb = mexp(p[2]), a1 = p[3], a2 = p[4];
+            T a = e(0), ph = t - p[1], tb = e(2), a1 = p[3], a2 = p[4];
             T ps = sp64_t(ph);
             T sp = mexp(ph) / (1.0 + mexp(ph));
             T lr = mlog(ps / tb);
@@ -200,6 +226,10 @@ __device__ inline void model_grad_t(int m, const T* p, T t, T* o) {
             return;
         }
     }
+}
+template <class T>
+__device__ inline void model_grad_t(int m, const T* p, T t, T* o) {
+    model_grad_e(m, p, ExpNow<T>{m, p}, t, o);
 }
 __device__ inline void model_grad_f64(int m, const double* p, double t, double* o) { model_grad_t<double>(m, p, t, o); }
 
