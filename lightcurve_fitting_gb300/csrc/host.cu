@@ -169,7 +169,8 @@ struct lcf_ctx {
     int cand_bps_rest[N_TUNE] = {1, 1, 1};  // blocks per SM, the other swarms
     int max_pso_warps_per_sm = 1;
     int lb_grid = 1;          // blocks of the persistent polish grid
-    int lb_n_long = 0;        // bands polished by a whole warp (LB_LONG_OBS observations or more)
+    int lb_n_long = 0;        // bands of LB_LONG_OBS observations or more
+    int lb_n_mid = 0;         // bands polished by a whole warp (polish_warp_obs observations or more)
     int cfg = 0;             // candidate of the current fit
     bool exploring = false;
     uint32_t bucket = 0;
@@ -530,7 +531,8 @@ static int prepare_layout(lcf_ctx* ctx, int n_sources, int n_bands, int64_t n_ob
     ctx->n_obs = n_obs;
     ctx->opts = o;
     int64_t n_max = 1;
-    int n_long = 0;
+    int n_long = 0, n_mid = 0;
+    const int warp_obs = polish_warp_obs(n_bands, ctx->lb_grid);
     for (int b = 0; b < n_bands; b++) {
         const int64_t nb_obs = ctx->h_boff[b + 1] - ctx->h_boff[b];
         n_max = std::max<int64_t>(n_max, nb_obs);
@@ -551,9 +553,11 @@ static int prepare_layout(lcf_ctx* ctx, int n_sources, int n_bands, int64_t n_ob
     rc |= grow(ctx, ctx->t64, no * 8);
     rc |= grow(ctx, ctx->f64, no * 8);
     rc |= grow(ctx, ctx->fe64, no * 8);
+        n_mid += nb_obs >= warp_obs ? 1 : 0;
     rc |= grow(ctx, ctx->var64, no * 8);
     rc |= grow(ctx, ctx->uf64, no * 8);
     rc |= grow(ctx, ctx->mag64, no * 8);
+    ctx->lb_n_mid = n_mid;
     rc |= grow(ctx, ctx->up, no);
     rc |= grow(ctx, ctx->ffa, no * sizeof(float4));
     rc |= grow(ctx, ctx->ffb, no * sizeof(float2));
@@ -741,6 +745,7 @@ static int prepare_layout(lcf_ctx* ctx, int n_sources, int n_bands, int64_t n_ob
     d.out = (BandOut*)ctx->out.p;
     d.mb = (MbState*)ctx->mb.p;
     for (int s = 0; s < 7; s++) {
+    d.num_sms = ctx->num_sms;
         d.tasks[s] = (PsoTask*)ctx->tasks[s].p;
         d.task_cap[s] = (int)ctx->task_cap[s];
     }
@@ -774,6 +779,7 @@ static int prepare_layout(lcf_ctx* ctx, int n_sources, int n_bands, int64_t n_ob
     d.mb_slot_base = (int64_t)n_bands * 32;
     d.smem_obs = ctx->smem_obs;
     d.wait_polls = ctx->wait_polls;
+    d.lb_n_mid = ctx->lb_n_mid;
     return 0;
 }
 

@@ -25,13 +25,19 @@
 // warp hold bands of similar length and their observation loops end
 // together.
 //
-// On a batch that fills the grid the polish is bound by instruction fetch
-// (its double-float terms and FP64 line search are long code; measured on
-// GB300, more resident warps at different points of it made it slower).  The
-// warps of a block then run a round in step: a block barrier before and
-// after the evaluation, so that they fetch the same code.  A smaller batch is
-// bound by the latency of its polishes, which the barriers would lengthen.  The group's scalar state and the per-lane
+// The polish is bound by instruction fetch (its double-float terms and FP64
+// line search are long code; measured on GB300, more resident warps at
+// different points of it made it slower, and a warp on its own spends ~15 us
+// on an observation's term).  The warps of a block run a round in step: a
+// block barrier before and after the evaluation, so that they fetch the same
+// code.  On small batches too: 1,000 uneven sources polish in 79 ms in step
+// and in 96 ms without the barriers.  The group's scalar state and the per-lane
 // vectors live in shared memory, leaving the registers to the evaluation.
+//
+// Where the batch leaves warps free, a band gets a whole warp: four
+// observations then go through the term for one fetch of it, and
+// add_round_v8 adds them in the eight lanes' order, so the result does not
+// depend on the batch.
 //
 // Arithmetic: the reference's algorithm in FP64 (lbfgs.cuh restates it for
 // one thread).  The dot products are sums over the eight lanes by xor 4, 2, 1
@@ -141,14 +147,51 @@ __device__ __noinline__ int group_fp64_terms(const double* t, const double* flux
     return nonfinite;
 }
 
+// The eight sums of a band that a whole warp evaluates in the eight-lane
+// order: lane v + 8 u holds the term vector v8 of the (4 r + u)-th observation
+// of sum lane v in round r.  The four lanes of a sum lane trade components
+// (xor 16, then xor 8), so that lane v + 8 u ends with components 2 u and
+// 2 u + 1 of all four observations, and adds them in the observations' order:
+// the bits of eight lanes that take four observations each, one after another.
+__device__ __forceinline__ void add_round_v8(const ff* v8, ff& s0, ff& s1) {
+    const int lane = threadIdx.x & 31;
+    const bool b4 = lane & 16, b3 = lane & 8;
+    ff own[4], oth[4];  // this lane's and its xor-16 partner's components 4 b4 .. 4 b4 + 3
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        own[i] = b4 ? v8[4 + i] : v8[i];
+        oth[i] = shfl_xor_ff_m(b4 ? v8[i] : v8[4 + i], 16, FULL);
+    }
+    ff p[2][4];  // [component][observation u]
+#pragma unroll
+    for (int c = 0; c < 2; c++) {
+        const ff a = b3 ? own[2 + c] : own[c], b = b3 ? oth[2 + c] : oth[c];
+        const ff ra = shfl_xor_ff_m(b3 ? own[c] : own[2 + c], 8, FULL);
+        const ff rb = shfl_xor_ff_m(b3 ? oth[c] : oth[2 + c], 8, FULL);
+        // observation u of lane bits (b4, b3): own a = (b4, b3), b = (!b4, b3), ra = (b4, !b3), rb = (!b4, !b3)
+        const ff x0 = b4 ? b : a, x2 = b4 ? a : b;      // u with bit 0 = b3
+        const ff y0 = b4 ? rb : ra, y2 = b4 ? ra : rb;  // u with bit 0 = !b3
+        p[c][0] = b3 ? y0 : x0;
+        p[c][1] = b3 ? x0 : y0;
+        p[c][2] = b3 ? y2 : x2;
+        p[c][3] = b3 ? x2 : y2;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        s0 = ff_add(s0, p[0][u]);
+        s1 = ff_add(s1, p[1][u]);
+    }
+}
+
 // Cost and projected gradient of the bounded problem (BoundedPsoCost,
 // src/parametric.rs:1500-1535) at the point whose component j is xj in lane
 // j of each group: PsoCost::cost_from_slice with the population prior and
 // the Villar constraint, and PsoCost::gradient.  G lanes a group (8, or 32:
-// the whole warp, whose four sets of eight lanes hold the same vectors).
+// the whole warp, whose four sets of eight lanes hold the same vectors); the
+// observations are summed in the order of V lanes (8 or 32).
 // Warp-collective (every lane calls it; a group with B.n == 0 evaluates
 // nothing of use).  Returns 1 when the group's terms ran in FP64.
-template <int MODEL, int G>
+template <int MODEL, int G, int V>
 __device__ __forceinline__ int group_cost_grad(const DeviceBatch& d, const GroupBand& B, double xj, bool want_grad,
                                                double& fo, double& gj) {
     constexpr int np = n_params_of(MODEL), se = se_idx_of(MODEL);
@@ -203,13 +246,38 @@ __device__ __forceinline__ int group_cost_grad(const DeviceBatch& d, const Group
         int redo = 0;
         const float4* fa = d.ffa + B.off;
         const float2* fb = d.ffb + B.off;
-        for (int i = lane & (G - 1); i < B.n; i += G)
-            ff_obs_term<MODEL>(fm, fa[i], fb[i], se2f, want_grad, nf, gf, nonfinite, redo);
+        ff s0 = ffm(0.0f, 0.0f), s1 = ffm(0.0f, 0.0f);
+        if constexpr (G == V) {
+            for (int i = lane & (G - 1); i < B.n; i += G)
+                ff_obs_term<MODEL>(fm, fa[i], fb[i], se2f, want_grad, nf, gf, nonfinite, redo);
+        } else {
+            for (int i0 = 0; i0 < B.n; i0 += 32) {
+                ff t[8];
+#pragma unroll
+                for (int k = 0; k < 8; k++) t[k] = ffm(0.0f, 0.0f);
+                if (i0 + lane < B.n)
+                    ff_obs_term<MODEL>(fm, fa[i0 + lane], fb[i0 + lane], se2f, want_grad, t[0], t + 1, nonfinite, redo);
+                add_round_v8(t, s0, s1);
+            }
+        }
         in_ff = __ballot_sync(gm, redo) == 0u;
         if (in_ff) {
             nonfinite = __ballot_sync(gm, nonfinite) != 0u;
             const ff v[8] = {nf, gf[0], gf[1], gf[2], gf[3], gf[4], gf[5], gf[6]};
-            if (G == 32) {  // lane l: the warp's total of v[(l >> 2) & 7]
+            if (G != V) {
+                // lane v + 8 u: the totals of components 2 u, 2 u + 1, summed as
+                // group_rs8_ff does (ff_add commutes)
+#pragma unroll
+                for (int k = 4; k; k >>= 1) {
+                    s0 = ff_add(s0, shfl_xor_ff_m(s0, k, FULL));
+                    s1 = ff_add(s1, shfl_xor_ff_m(s1, k, FULL));
+                }
+                const double t0s = ff_to(s0), t1s = ff_to(s1);
+                nsum = __shfl_sync(FULL, t0s, 0);
+                const int src = 8 * (((j + 1) & 7) >> 1);
+                const double ge = __shfl_sync(FULL, t0s, src), go = __shfl_sync(FULL, t1s, src);
+                gs = ((j + 1) & 1) ? go : ge;
+            } else if (G == 32) {  // lane l: the warp's total of v[(l >> 2) & 7]
                 const double tot = ff_to(reduce_scatter8_ff(v));
                 nsum = __shfl_sync(FULL, tot, 0);
                 gs = __shfl_sync(FULL, tot, (4 * (1 + j)) & 31);
@@ -230,10 +298,11 @@ __device__ __forceinline__ int group_cost_grad(const DeviceBatch& d, const Group
         }
         const double se2 = ep[se] * ep[se];
         const int64_t o = B.off;
-        const int nf64 = group_fp64_terms<MODEL, G>(d.t64 + o, d.f64 + o, d.var64 + o, d.uf64 + o, d.up + o, B.n, q,
+        // (a warp summing in the eight-lane order: each set of eight lanes does it all)
+        const int nf64 = group_fp64_terms<MODEL, V>(d.t64 + o, d.f64 + o, d.var64 + o, d.uf64 + o, d.up + o, B.n, q,
                                                     ep, rp, se2, want_grad, v);
         nonfinite = __ballot_sync(gm, nf64) != 0u;
-        if (G == 32) {
+        if (V == 32) {
             const double tot = reduce_scatter8(v);
             nsum = __shfl_sync(FULL, tot, 0);
             gs = __shfl_sync(FULL, tot, (4 * (1 + j)) & 31);
@@ -271,17 +340,15 @@ enum LbPhase : int {
 };
 
 // Polishes the queued bands of MODEL with G lanes a band (8: four bands a
-// warp; 32: one): d.polish_order[i] for the indices i in [lo, hi) that this
-// warp's groups take from the queue counter `next`.  `lockstep` (uniform
-// over the grid): the block's warps run each round in step.
-// Out of line: the two instantiations of a model (8 and 32 lanes a band)
-// then take their registers separately.
+// warp; 32: one), summing in the order of V lanes: d.polish_order[i] for the indices i in [lo, hi) that this
+// warp's groups take from the queue counter `next`, the block's warps running
+// each round in step.
+// Out of line: the instantiations of a model then take their registers separately.
 #ifndef LCF_LB_QUEUE_ATTR
 #define LCF_LB_QUEUE_ATTR __noinline__
 #endif
-template <int MODEL, int G>
-__device__ LCF_LB_QUEUE_ATTR void polish_queue(const DeviceBatch& d, LbWarpShared& sh, int lo, int hi, int* next,
-                                               bool lockstep) {
+template <int MODEL, int G, int V>
+__device__ LCF_LB_QUEUE_ATTR void polish_queue(const DeviceBatch& d, LbWarpShared& sh, int lo, int hi, int* next) {
     constexpr int np = n_params_of(MODEL), t0i = t0_idx_of(MODEL), M = 7, MAXIT = 50;
     const double ftol = 1e-4, gtol = 0.9, xtol = 1e-10, xtrapf = 4.0, stpmin = 0.0, stpmax = INFINITY;
     const double tol_grad = 1e-6, tol_cost = 2.220446049250313e-16;
@@ -392,7 +459,7 @@ __device__ LCF_LB_QUEUE_ATTR void polish_queue(const DeviceBatch& d, LbWarpShare
         // in step, the block's warps evaluate together (see the header): a
         // barrier before and after the evaluation
         const bool active = phase != LB_DONE;
-        if (lockstep ? !__syncthreads_or(active) : !__any_sync(FULL, active)) break;
+        if (!__syncthreads_or(active)) break;
         if constexpr (MODEL == METZGER) continue;  // never polished (every group is done)
         const bool want_grad = phase == LB_START || phase == LB_LS;
         GroupBand B;
@@ -405,8 +472,8 @@ __device__ LCF_LB_QUEUE_ATTR void polish_queue(const DeviceBatch& d, LbWarpShare
         B.hi_j = hi_j;
         double fe = 0.0, ge = 0.0;
         int used64 = 0;
-        if (__any_sync(FULL, active)) used64 = group_cost_grad<MODEL, G>(d, B, xe, want_grad, fe, ge);
-        if (lockstep) __syncthreads();
+        if (__any_sync(FULL, active)) used64 = group_cost_grad<MODEL, G, V>(d, B, xe, want_grad, fe, ge);
+        __syncthreads();
         if (!active) continue;
         fp64_evals += used64;
         // the transition of this group's phase; the steps shared by several

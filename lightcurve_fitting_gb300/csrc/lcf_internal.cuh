@@ -236,6 +236,7 @@ struct Counters {
 struct DeviceBatch {
     // raw inputs (FP64, caller layout)
     const double* times;
+    int32_t lb_next_mid[8];     // per model: next index of its middle bands (a warp a band, eight-lane order)
     const double* flux;
     const double* err;
     const int64_t* band_off;
@@ -248,6 +249,7 @@ struct DeviceBatch {
     double* t64;            // [n_obs] sorted FP64 copies for the FP64 stages
     double* f64;            // flux / peak
     double* fe64;           // err / peak
+    int num_sms;
     double* var64;          // obs_var
     double* uf64;           // upper flux
     double* mag64;          // observed magnitude
@@ -285,6 +287,7 @@ struct DeviceBatch {
     float* scratch_svi;     // MetzgerKN SVI scratch, 20 values per observation
     double* t0_state;       // per band: t0_min, t0_max, best t0 of the profile search
     int64_t t0_slot_base;   // first PsoResult slot of the t0 search region
+    int lb_n_mid;           // bands polished by a whole warp (the first of polish_order; >= lb_n_long)
     int64_t mb_slot_base;   // first PsoResult slot of the MultiBazin region
     int smem_obs;           // observations staged per warp in the PSO kernel
     int wait_polls;         // bound of the staging copy's barrier wait, in polls (lcf_set_wait_bound)
@@ -339,6 +342,9 @@ void launch_select(const DeviceBatch& d, int fit_all, int forced, cudaStream_t s
 void launch_svi(const DeviceBatch& d, cudaStream_t s);
 // one SVI step's ELBO estimate and gradient at given variational parameters
 // (lcf_svi_elbo_grad); scratch = 5 n floats per point
+// Bands of at least this many observations (a multiple of 8, at most
+// LB_LONG_OBS) are polished by a whole warp.
+int polish_warp_obs(int n_bands, int lb_grid);
 void launch_svi_grad(int model, const float4* obs, int n, float t_last, const double* init, const double* vpar,
                      int n_points, const double* eps, int n_samples, double* elbo, double* grad, int* flags,
                      float* scratch, cudaStream_t s);

@@ -42,37 +42,36 @@ namespace lcf {
 #ifndef LCF_LB_BLOCK
 #define LCF_LB_BLOCK 256
 #endif
-// Each model's queue in two parts: its first n_long bands (the longest) with
-// a warp a band, the rest with eight lanes a band.
+// Each model's queue in three parts: its first n_long bands (the longest) with
+// a warp a band, the bands up to n_mid with a warp a band in the eight-lane
+// order of summation, and the rest with eight lanes a band.
 template <int MODEL>
-__device__ __forceinline__ void polish_model(const DeviceBatch& d, LbWarpShared& w, int n_long, bool lockstep) {
-    polish_queue<MODEL, 32>(d, w, 0, n_long, &d.ctr->lb_next_long[MODEL], lockstep);
-    polish_queue<MODEL, 8>(d, w, n_long, d.n_bands, &d.ctr->lb_next[MODEL], lockstep);
+__device__ __forceinline__ void polish_model(const DeviceBatch& d, LbWarpShared& w, int n_long, int n_mid) {
+    polish_queue<MODEL, 32, 32>(d, w, 0, n_long, &d.ctr->lb_next_long[MODEL]);
+    polish_queue<MODEL, 32, 8>(d, w, n_long, n_mid, &d.ctr->lb_next_mid[MODEL]);
+    polish_queue<MODEL, 8, 8>(d, w, n_mid, d.n_bands, &d.ctr->lb_next[MODEL]);
 }
 
-// `stagger`: block k starts at model 8k / gridDim.x and takes the models in
-// turn from there, and the warps of a block do not run in step: a batch with
-// fewer bands than the grid has polish slots runs the eight models' queues
-// at once.  Otherwise every block takes the models in order, its warps in
-// step, and the warps of an SM share one model's code.
+// `stagger`: SM k's blocks start at model 8k / num_sms and take the models in
+// turn from there (blocks k and k + num_sms share an SM, and so a model's
+// code).  Otherwise every block takes the models in order.
 __global__ void __launch_bounds__(LCF_LB_BLOCK, LCF_LB_MINB)
-    lbfgs_kernel(DeviceBatch d, int model_mask, int stagger, int n_long) {
+    lbfgs_kernel(DeviceBatch d, int model_mask, int stagger, int n_long, int n_mid) {
     extern __shared__ LbWarpShared lb_sh[];
     LbWarpShared& w = lb_sh[threadIdx.x >> 5];
-    const int start = stagger ? (int)((8ll * blockIdx.x) / gridDim.x) : 0;
-    const bool lockstep = !stagger;
+    const int start = stagger ? (int)((8ll * (blockIdx.x % d.num_sms)) / d.num_sms) : 0;
     for (int k = 0; k < 8; k++) {
         const int m = (start + k) & 7;
         if (!((model_mask >> m) & 1)) continue;
         switch (m) {
-            case BAZIN: polish_model<BAZIN>(d, w, n_long, lockstep); break;
-            case VILLAR: polish_model<VILLAR>(d, w, n_long, lockstep); break;
-            case TDE: polish_model<TDE>(d, w, n_long, lockstep); break;
-            case ARNETT: polish_model<ARNETT>(d, w, n_long, lockstep); break;
-            case MAGNETAR: polish_model<MAGNETAR>(d, w, n_long, lockstep); break;
-            case SHOCK: polish_model<SHOCK>(d, w, n_long, lockstep); break;
-            case AFTERGLOW: polish_model<AFTERGLOW>(d, w, n_long, lockstep); break;
-            default: polish_model<METZGER>(d, w, n_long, lockstep); break;
+            case BAZIN: polish_model<BAZIN>(d, w, n_long, n_mid); break;
+            case VILLAR: polish_model<VILLAR>(d, w, n_long, n_mid); break;
+            case TDE: polish_model<TDE>(d, w, n_long, n_mid); break;
+            case ARNETT: polish_model<ARNETT>(d, w, n_long, n_mid); break;
+            case MAGNETAR: polish_model<MAGNETAR>(d, w, n_long, n_mid); break;
+            case SHOCK: polish_model<SHOCK>(d, w, n_long, n_mid); break;
+            case AFTERGLOW: polish_model<AFTERGLOW>(d, w, n_long, n_mid); break;
+            default: polish_model<METZGER>(d, w, n_long, n_mid); break;
         }
     }
 }
@@ -89,13 +88,27 @@ int lbfgs_grid(int num_sms) {
 
 void launch_lbfgs(const DeviceBatch& d, int model_mask, cudaStream_t s) {
     if (d.n_bands == 0) return;
-    // a warp a band for the bands of LB_LONG_OBS observations or more (the
-    // polish of a long band on eight lanes would set the kernel's tail).  The
-    // split depends on the band alone, not on the batch: a band's summation
-    // order, and so its fit, is the same in any batch.
-    const int64_t warps = (int64_t)d.lb_grid * (LCF_LB_BLOCK / 32);
-    lbfgs_kernel<<<d.lb_grid, LCF_LB_BLOCK, LB_SMEM, s>>>(d, model_mask, (int64_t)d.n_bands < 4 * warps ? 1 : 0,
-                                                          d.lb_n_long);
+// A batch of fewer bands than five per warp of the grid waits for its longest
+// polishes: every band then gets a warp, and the SMs start at staggered models
+// so that the models' queues drain together.  Larger batches are bound by
+// instruction fetch: eight lanes a band below 96 observations, where the
+// state machine outweighs the observations, and all blocks on one model.
+// Polish ms (GB300, uneven batches of 1,000 / 2,500 / 3,500 / 6,000 / 10,000
+// sources): every band a warp 79 / 161 / 222 / 405 / 644, from 96
+// observations on 100 / 188 / 244 / 328 / 500, eight lanes below 256 for all
+// 162 / - / - / - / 518.
+static bool polish_small(int n_bands, int lb_grid) {
+    return (int64_t)n_bands < 5ll * lb_grid * (LCF_LB_BLOCK / 32);
+}
+int polish_warp_obs(int n_bands, int lb_grid) {
+    return polish_small(n_bands, lb_grid) ? 0 : 96;
+}
+
+    // The bands of LB_LONG_OBS observations or more are summed in the order of
+    // 32 lanes, the others in that of eight, whatever the batch and however
+    // many lanes evaluate them: a band's fit is the same in any batch.
+    lbfgs_kernel<<<d.lb_grid, LCF_LB_BLOCK, LB_SMEM, s>>>(d, model_mask, polish_small(d.n_bands, d.lb_grid),
+                                                          d.lb_n_long, d.lb_n_mid);
 }
 
 // The polish queue's band order: longest first (counting sort on 256 keys,
