@@ -13,7 +13,10 @@
 // reduced across the warp.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "lcf_internal.cuh"
+#include "metzger_block.cuh"
 #include "models_f32.cuh"
 #include "models_f64.cuh"
 
@@ -139,14 +142,13 @@ __device__ double band_ll_w(int m, const BandView& b, const double* p, double* s
 // 0.5 apart and pick grid points, so FP32 prediction rounding (1e-7
 // relative) moves no decision except a value within ~1e-5 of a threshold.
 // ---------------------------------------------------------------------------
-__device__ void scan_constants(const BandView& b, double se2, double* cst) {
-    for (int i = threadIdx.x & 31; i < b.n; i += 32) {
+__device__ void scan_constants(const BandView& b, double se2, double* cst, int i0, int stride) {
+    for (int i = i0; i < b.n; i += stride) {
         double tv = b.var[i] + se2;
         cst[3 * i] = 1.0 / tv;
         cst[3 * i + 1] = 1.0 / sqrt(tv);
         cst[3 * i + 2] = log(2.0 * 3.14159265358979323846 * tv);
     }
-    __syncwarp();
 }
 
 // FP32 prediction -> FP64 value; false for a prediction the reference finds
@@ -232,12 +234,8 @@ __device__ void shape_sums_fast(int m, const double* p, const float4* obs, const
 }
 
 // ---------------------------------------------------------------------------
-// MetzgerKN refinement scans, one scan point per lane.  The scans evaluate
-// up to ~140 independent parameter vectors per band; each lane integrates
-// its own vector's ODE (FP64, metzger_sweep64 — the arithmetic of
-// metzger_f64) twice: the first sweep finds the peak the predictions are
-// normalised by (and the largest detection prediction for the rescale), the
-// second forms the band's terms in observation order.
+// MetzgerKN refinement scans: a block per band, one scan point per lane
+// (metzger_block.cuh).
 // ---------------------------------------------------------------------------
 struct MzPeak {
     const uint8_t* up;
@@ -250,7 +248,7 @@ struct MzPeak {
 struct MzLl {
     const BandView* b;
     const double* cst;
-    double inv_peak, scale, ll;
+    double scale, ll;
     __device__ void term(int j, double pr) {
         if (!isfinite(pr)) return;
         const double* c = cst + 3 * j;
@@ -261,51 +259,21 @@ struct MzLl {
             ll += -0.5 * (r * r * c[0] + c[2]);
         }
     }
-    __device__ void operator()(int j, double l) { term(j, l * inv_peak * scale); }
 };
 
-// Bands of at most MZ_KEEP observations keep the first sweep's interpolants
-// in shared memory (lane-interleaved: entry j of a lane at keep[32 j]) and
-// form the terms from them, in the second sweep's order, instead of
-// integrating the ODE again; longer bands sweep twice.
-constexpr int MZ_KEEP = 32;
-struct MzKeep {
-    const uint8_t* up;
-    double* keep;
-    double mx;
-    __device__ void operator()(int j, double l) {
-        if (!up[j]) mx = fmax(mx, l);
-        keep[32 * j] = l;
-    }
-};
-__device__ __forceinline__ bool metzger_first_sweep(const double* p, const BandView& b, double* keep, double& mx,
-                                                    int& j_start, double& l_peak) {
-    if (keep) {
-        MzKeep kp{b.up, keep, -INFINITY};
-        bool ok = metzger_sweep64(p, b.t, b.n, kp, j_start, l_peak);
-        mx = kp.mx;
-        return ok;
-    }
-    MzPeak pk{b.up, -INFINITY};
-    bool ok = metzger_sweep64(p, b.t, b.n, pk, j_start, l_peak);
-    mx = pk.mx;
-    return ok;
-}
-
-// band_ll_w for MetzgerKN by one lane (rescale: the PSO cost's peak rescale);
-// keep: this lane's interpolant slots (nullptr: sweep twice)
-__device__ double metzger_ll_lane(const double* p, const BandView& b, const double* cst, bool rescale,
-                                  double* keep) {
-    if (b.n > MZ_KEEP) keep = nullptr;
-    MzPeak pk{b.up, -INFINITY};
-    int j_start;
+// band_ll_w for MetzgerKN by one lane (rescale: the PSO cost's peak rescale)
+__device__ double metzger_ll_lane(MzTables& T, int slot, int col, const double* p, const BandView& b,
+                                  const double* cst, bool rescale) {
+    int j_start = b.n;
     double l_peak;
-    bool ok = metzger_first_sweep(p, b, keep, pk.mx, j_start, l_peak);
+    bool ok = mz_sweep(T, p, slot, col, l_peak);
     bool valid = ok && l_peak > 0.0 && isfinite(l_peak);
     double scale = 1.0;
     if (rescale) {
         // largest normalised detection prediction; invalid sweeps and the
         // observations before t0 predict 0
+        MzPeak pk{b.up, -INFINITY};
+        if (valid) mz_visit(T, slot, col, p[3], b.t, b.n, j_start, pk);
         double mx = -INFINITY;
         int z_end = valid ? j_start : b.n;
         for (int j = 0; j < z_end; j++)
@@ -313,39 +281,36 @@ __device__ double metzger_ll_lane(const double* p, const BandView& b, const doub
         if (valid) mx = fmax(mx, pk.mx / l_peak);
         if (mx > 1e-10 && isfinite(mx)) scale = fmin(fmax(1.0 / mx, 0.1), 10.0);
     }
-    MzLl acc{&b, cst, valid ? 1.0 / l_peak : 0.0, scale, 0.0};
+    MzLl acc{&b, cst, scale, 0.0};
+    if (valid) {
+        j_start = 0;
+        while (j_start < b.n && b.t[j_start] - p[3] <= 0.0) j_start++;
+    }
     int z_end = valid ? j_start : b.n;
     for (int j = 0; j < z_end; j++) acc.term(j, 0.0 * scale);
     if (valid) {
-        // the same interpolants, normalised
+        // the interpolants, normalised
         struct Norm {
             MzLl* a;
             double lpk;
             __device__ void operator()(int j, double l) { a->term(j, l / lpk * a->scale); }
         } nv{&acc, l_peak};
-        if (keep) {
-            for (int j = j_start; j < b.n; j++) nv(j, keep[32 * j]);
-        } else {
-            int js;
-            double lp;
-            metzger_sweep64(p, b.t, b.n, nv, js, lp);
-        }
+        mz_visit(T, slot, col, p[3], b.t, b.n, j_start, nv);
     }
     return acc.ll;
 }
 
 // shape sums of profile_t0_refine for MetzgerKN by one lane: sw, sy, sf,
 // syf, sff over detections of the normalised prediction
-__device__ void metzger_shape_lane(const double* p, const BandView& b, const double* cst, double* s5, double* keep) {
-    if (b.n > MZ_KEEP) keep = nullptr;
-    double mx_unused;
+__device__ void metzger_shape_lane(MzTables& T, int slot, int col, const double* p, const BandView& b,
+                                   const double* cst, double* s5) {
     int j_start;
     double l_peak;
-    bool ok = metzger_first_sweep(p, b, keep, mx_unused, j_start, l_peak);
+    bool ok = mz_sweep(T, p, slot, col, l_peak);
     bool valid = ok && l_peak > 0.0 && isfinite(l_peak);
     double sw = 0, sy = 0, sf = 0, syf = 0, sff = 0;
-    int z_end = valid ? j_start : b.n;
-    for (int j = 0; j < z_end; j++) {
+    for (int j = 0; j < b.n; j++) {
+        if (valid && !(b.t[j] - p[3] <= 0.0)) break;
         if (b.up[j]) continue;
         double w = cst[3 * j];
         sw += w; sy += w * b.f[j];
@@ -363,109 +328,186 @@ __device__ void metzger_shape_lane(const double* p, const BandView& b, const dou
                 sw += w; sy += w * fj; sf += w * sh; syf += w * fj * sh; sff += w * sh * sh;
             }
         } su{&b, cst, l_peak, sw, sy, sf, syf, sff};
-        if (keep) {
-            for (int j = j_start; j < b.n; j++) su(j, keep[32 * j]);
-        } else {
-            int js;
-            double lp;
-            metzger_sweep64(p, b.t, b.n, su, js, lp);
-        }
+        mz_visit(T, slot, col, p[3], b.t, b.n, j_start, su);
         sw = su.sw; sy = su.sy; sf = su.sf; syf = su.syf; sff = su.sff;
     }
     s5[0] = sw; s5[1] = sy; s5[2] = sf; s5[3] = syf; s5[4] = sff;
 }
 
-// profile_t0_refine + profile_refine_all for a MetzgerKN band (np = 5,
-// t0 = p[3], sigma_extra = p[4]; no baseline parameter), lanes over scan
-// points; the sequential decisions run uniformly on the gathered values.
-__device__ void refine_metzger(const BandStats& bs, const BandView& b, const double* cst, double* mu, double* ls,
-                               double* keep) {
+// Magnitude-space chi2 of a MetzgerKN band by one warp: the prediction at mu
+// (table 0), or at the PSO parameters where fewer than half are positive.
+__device__ double metzger_mag_chi2(MzTables& T, const BandStats& bs, const BandView& b, const BandOut& o,
+                                   const double* mu) {
     const int lane = threadIdx.x & 31;
-    constexpr int m = METZGER, np = 5, se = 4, t0i = 3, NG = 25;
-    double t0_lo = bs.t_first - 30.0, t0_hi = bs.t_peak_all + 5.0;
-    if (t0_lo < t0_hi) {
-        auto grid = [&](int gi) { return t0_lo + (t0_hi - t0_lo) * (double)gi / (double)(NG - 1); };
-        // profiled amplitude at each grid t0, then its log-likelihood (rescaled)
-        double my_ll = -INFINITY;
-        if (lane < NG) {
-            double p[MAXP];
-            for (int j = 0; j < np; j++) p[j] = mu[j];
-            p[t0i] = grid(lane);
-            double saved_la = p[0];
-            p[0] = 0.0;
-            double s5[5];
-            metzger_shape_lane(p, b, cst, s5, keep);
-            double syf = s5[3], sff = s5[4];
-            if (sff > 1e-20 && syf / sff > 1e-10) p[0] = log(syf / sff);
-            else p[0] = saved_la;
-            my_ll = metzger_ll_lane(p, b, cst, true, keep);
-        }
-        double best_t0 = mu[t0i], best_ll = -INFINITY;
-        for (int gi = 0; gi < NG; gi++) {
-            double l = __shfl_sync(FULL, my_ll, gi);
-            if (l > best_ll) { best_ll = l; best_t0 = grid(gi); }
-        }
-        // log-likelihood at mu with t0 on each grid point (no rescale)
-        double e_ll = -INFINITY;
-        if (lane < NG) {
-            double p[MAXP];
-            for (int j = 0; j < np; j++) p[j] = mu[j];
-            p[t0i] = grid(lane);
-            e_ll = metzger_ll_lane(p, b, cst, false, keep);
-        }
-        double lo1 = best_t0, hi1 = best_t0, thr = best_ll - 0.5;
-        for (int gi = NG - 1; gi >= 0; gi--) {
-            double t0 = grid(gi);
-            double l = __shfl_sync(FULL, e_ll, gi);
-            if (t0 >= best_t0) continue;
-            if (l >= thr) lo1 = t0;
-            else break;
-        }
-        for (int gi = 0; gi < NG; gi++) {
-            double t0 = grid(gi);
-            double l = __shfl_sync(FULL, e_ll, gi);
-            if (t0 <= best_t0) continue;
-            if (l >= thr) hi1 = t0;
-            else break;
-        }
-        mu[t0i] = best_t0;
-        ls[t0i] = log(fmax((hi1 - lo1) / 2.0, 0.1));
+    constexpr int np = 5, PSO_SLOT = 24;
+    double l_peak;
+    int valid = 0, slot = 0, col = 62;
+    const double* use = mu;
+    auto sweep = [&]() {
+        int v = 0;
+        if (lane == 0) v = mz_sweep(T, use, slot, col, l_peak) && !(l_peak <= 0.0 || !isfinite(l_peak));
+        __syncwarp();
+        l_peak = __shfl_sync(FULL, l_peak, 0);
+        valid = __shfl_sync(FULL, v, 0);
+    };
+    auto pred = [&](int i) {
+        const double ph = b.t[i] - use[3];
+        if (!valid || ph <= 0.0) return 0.0;
+        int g = 0;
+        for (int step = 128; step; step >>= 1)
+            if (g + step <= MZ_NG && ph > T.row[g + step - 1][0][slot]) g += step;
+        return mz_interp(T, slot, col, ph, g) / l_peak;
+    };
+    sweep();
+    int npos = 0;
+    for (int i = lane; i < b.n; i += 32) npos += (pred(i) * b.peak > 0.0) ? 1 : 0;
+    for (int k = 16; k; k >>= 1) npos += __shfl_xor_sync(FULL, npos, k);
+    double pso[MAXP];
+    // the joint fit always takes mu (src/parametric.rs:4057-4073)
+    if (npos < b.n / 2 && !bs.joint) {
+        for (int j = 0; j < np; j++) pso[j] = o.pso_params[j];
+        use = pso;
+        slot = PSO_SLOT;
+        col = 63;
+        __syncwarp();
+        mz_tabulate(T, 1, bs.t_last, [&](int) { return pso[3]; }, lane, 32, PSO_SLOT);
+        __syncwarp();
+        sweep();
     }
-    // profile_refine_all: evaluation 0 = mu, 1 + 15 j + gi = parameter j on
-    // grid point gi; two rounds of 32 lanes
-    constexpr int NE = 1 + 4 * 15;
-    double r_ll[2];
-    for (int round = 0; round < 2; round++) {
-        int e = round * 32 + lane;
-        r_ll[round] = -INFINITY;
-        if (e < NE) {
+    double msum = 0.0;
+    int mcount = 0;
+    for (int i = lane; i < b.n; i += 32) {
+        double pf = pred(i) * b.peak;
+        if (pf > 0.0 && b.f[i] > 0.0) {
+            double mpred = -2.5 * log10(pf) + 23.9;
+            double merr = 1.0857 * b.fe[i] / b.f[i];
+            if (merr > 0.0) {
+                double r = b.mag[i] - mpred;
+                msum += r * r / (merr * merr);
+                mcount++;
+            }
+        }
+    }
+    msum = wsum(msum);
+    for (int k = 16; k; k >>= 1) mcount += __shfl_xor_sync(FULL, mcount, k);
+    return mcount > 0 ? msum / (double)mcount : NAN;
+}
+
+// profile_t0_refine, profile_refine_all and the magnitude chi2 of the
+// MetzgerKN bands (np = 5, t0 = p[3], sigma_extra = p[4]; no baseline
+// parameter).  The sequential decisions run uniformly on the gathered values.
+// On the t0 grid warp 0 takes the profiled amplitude and its likelihood while
+// warp 1 takes the likelihoods at mu; then warps 0 and 1 take the 61
+// all-parameter points while warp 2 takes the magnitude chi2.  Bound by the
+// FP64 pipe.  The refinements of 600 bands x 8 models, GB300: 70 ms with a warp
+// a MetzgerKN band, each lane integrating its own ODE twice; 21 ms now.
+__global__ void __launch_bounds__(MZ_BLOCK) refine_metzger_kernel(DeviceBatch d) {
+    extern __shared__ __align__(16) unsigned char mz_raw[];
+    MzTables& T = *reinterpret_cast<MzTables*>(mz_raw);
+    __shared__ double s_ll[MZ_LANES], s_ell[32], s_mag;
+    constexpr int m = METZGER, np = 5, se = 4, t0i = 3, NG = 25, NE = 1 + 4 * 15;
+    static_assert(NG <= MZ_SLOTS && NE < 62 && 1 + 15 <= 24, "MetzgerKN scan tables");
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int n_metzger = d.ctr->band_hist[0];  // band_order's first (band_order_kernel)
+    for (int ib = blockIdx.x; ib < n_metzger; ib += gridDim.x) {
+        const int band = d.band_order[ib];
+        const BandStats bs = d.stats[band];
+        BandOut& o = d.out[band];
+        const BandView b = band_view(d, bs);
+        double* cst = d.scratch64 + 5 * bs.off;
+        double mu[MAXP], ls[MAXP];
+        for (int j = 0; j < np; j++) { mu[j] = o.mu[j]; ls[j] = o.log_sigma[j]; }
+        scan_constants(b, exp(2.0 * mu[se]), cst, tid, MZ_BLOCK);
+        const double t0_lo = bs.t_first - 30.0, t0_hi = bs.t_peak_all + 5.0;
+        if (t0_lo < t0_hi) {
+            auto grid = [&](int gi) { return t0_lo + (t0_hi - t0_lo) * (double)gi / (double)(NG - 1); };
+            mz_tabulate(T, NG, bs.t_last, grid, tid, MZ_BLOCK);
+            __syncthreads();
+            if (warp < 2 && lane < NG) {
+                double p[MAXP];
+                for (int j = 0; j < np; j++) p[j] = mu[j];
+                p[t0i] = grid(lane);
+                if (warp == 0) {
+                    // profiled amplitude at each grid t0, then its log-likelihood (rescaled)
+                    double saved_la = p[0];
+                    p[0] = 0.0;
+                    double s5[5];
+                    metzger_shape_lane(T, lane, lane, p, b, cst, s5);
+                    double syf = s5[3], sff = s5[4];
+                    if (sff > 1e-20 && syf / sff > 1e-10) p[0] = log(syf / sff);
+                    else p[0] = saved_la;
+                    s_ll[lane] = metzger_ll_lane(T, lane, lane, p, b, cst, true);
+                } else {
+                    // log-likelihood at mu with t0 on each grid point (no rescale)
+                    s_ell[lane] = metzger_ll_lane(T, lane, 32 + lane, p, b, cst, false);
+                }
+            }
+            __syncthreads();
+            double best_t0 = mu[t0i], best_ll = -INFINITY;
+            for (int gi = 0; gi < NG; gi++) {
+                double l = s_ll[gi];
+                if (l > best_ll) { best_ll = l; best_t0 = grid(gi); }
+            }
+            double lo1 = best_t0, hi1 = best_t0, thr = best_ll - 0.5;
+            for (int gi = NG - 1; gi >= 0; gi--) {
+                double t0 = grid(gi);
+                if (t0 >= best_t0) continue;
+                if (s_ell[gi] >= thr) lo1 = t0;
+                else break;
+            }
+            for (int gi = 0; gi < NG; gi++) {
+                double t0 = grid(gi);
+                if (t0 <= best_t0) continue;
+                if (s_ell[gi] >= thr) hi1 = t0;
+                else break;
+            }
+            mu[t0i] = best_t0;
+            ls[t0i] = log(fmax((hi1 - lo1) / 2.0, 0.1));
+        }
+        __syncthreads();
+        // profile_refine_all: evaluation 0 = mu, 1 + 15 j + gi = parameter j
+        // on grid point gi; table 0 = mu's t0, 1 + gi = t0's grid
+        auto scan = [&](int j, int gi) {
+            double slo = c_lo[m][j], shi = c_hi[m][j];
+            return slo + (shi - slo) * (double)gi / 14.0;
+        };
+        mz_tabulate(T, 16, bs.t_last, [&](int k) { return k == 0 ? mu[t0i] : scan(t0i, k - 1); }, tid, MZ_BLOCK);
+        __syncthreads();
+        if (tid < NE) {
             double p[MAXP];
             for (int k = 0; k < np; k++) p[k] = mu[k];
-            if (e > 0) {
-                int j = (e - 1) / 15, gi = (e - 1) % 15;
-                double slo = c_lo[m][j], shi = c_hi[m][j];
-                p[j] = slo + (shi - slo) * (double)gi / 14.0;
+            int slot = 0;
+            if (tid > 0) {
+                int j = (tid - 1) / 15, gi = (tid - 1) % 15;
+                p[j] = scan(j, gi);
+                if (j == t0i) slot = 1 + gi;
             }
-            r_ll[round] = metzger_ll_lane(p, b, cst, false, keep);
+            s_ll[tid] = metzger_ll_lane(T, slot, tid, p, b, cst, false);
         }
-    }
-    auto get = [&](int e) {
-        double a = __shfl_sync(FULL, r_ll[0], e & 31), c = __shfl_sync(FULL, r_ll[1], e & 31);
-        return e < 32 ? a : c;
-    };
-    double thr = get(0) - 0.5;
-    for (int j = 0; j < np; j++) {
-        if (j == se) continue;
-        double mu_j = mu[j], svi_sigma = exp(ls[j]);
-        double slo = c_lo[m][j], shi = c_hi[m][j];
-        if (shi - slo < 1e-10) continue;
-        double l1 = mu_j, h1 = mu_j;
-        for (int gi = 0; gi < 15; gi++) {
-            double val = slo + (shi - slo) * (double)gi / 14.0;
-            if (get(1 + j * 15 + gi) >= thr) { l1 = fmin(l1, val); h1 = fmax(h1, val); }
+        if (warp == 2) {
+            const double mc = metzger_mag_chi2(T, bs, b, o, mu);
+            if (lane == 0) s_mag = mc;
         }
-        double prof = fmax((h1 - l1) / 2.0, 1e-6);
-        ls[j] = log(fmax(fmax(svi_sigma, prof), c_pop_w[m][j]));
+        __syncthreads();
+        if (tid == 0) {
+            double thr = s_ll[0] - 0.5;
+            for (int j = 0; j < np; j++) {
+                if (j == se) continue;
+                double mu_j = mu[j], svi_sigma = exp(ls[j]);
+                double slo = c_lo[m][j], shi = c_hi[m][j];
+                if (shi - slo < 1e-10) continue;
+                double l1 = mu_j, h1 = mu_j;
+                for (int gi = 0; gi < 15; gi++) {
+                    double val = scan(j, gi);
+                    if (s_ll[1 + j * 15 + gi] >= thr) { l1 = fmin(l1, val); h1 = fmax(h1, val); }
+                }
+                double prof = fmax((h1 - l1) / 2.0, 1e-6);
+                ls[j] = log(fmax(fmax(svi_sigma, prof), c_pop_w[m][j]));
+            }
+            for (int j = 0; j < np; j++) { o.mu[j] = mu[j]; o.log_sigma[j] = ls[j]; }
+            o.mag_chi2 = s_mag;
+        }
+        __syncthreads();
     }
 }
 
@@ -528,46 +570,42 @@ __device__ __forceinline__ int band_order_key(const DeviceBatch& d, int b) {
     if (!d.stats[b].valid || m < 0) return 8;
     return m == METZGER ? 0 : 1 + m;
 }
-__global__ void band_hist_kernel(DeviceBatch d) {
-    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < d.n_bands; b += gridDim.x * blockDim.x)
-        atomicAdd(&d.ctr->band_hist[band_order_key(d, b)], 1);
-}
-__global__ void band_scan_kernel(DeviceBatch d) {  // one thread
-    int run = 0;
-    for (int k = 0; k < 9; k++) {
-        const int v = d.ctr->band_hist[k];
-        d.ctr->band_hist[k] = run;
-        run += v;
+// One block: the list is a few reads a band, less than two more launches.  On
+// return band_hist[0] is the number of MetzgerKN bands (band_order's first).
+constexpr int BO_BLOCK = 1024;
+__global__ void __launch_bounds__(BO_BLOCK) band_order_kernel(DeviceBatch d) {
+    __shared__ int pos[9];
+    const int tid = threadIdx.x;
+    if (tid < 9) pos[tid] = 0;
+    __syncthreads();
+    for (int b = tid; b < d.n_bands; b += BO_BLOCK) atomicAdd(&pos[band_order_key(d, b)], 1);
+    __syncthreads();
+    if (tid == 0) {
+        int run = 0;
+        for (int k = 0; k < 9; k++) {
+            const int v = pos[k];
+            d.ctr->band_hist[k] = v;
+            pos[k] = run;
+            run += v;
+        }
     }
-}
-__global__ void band_scatter_kernel(DeviceBatch d) {
-    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < d.n_bands; b += gridDim.x * blockDim.x)
-        d.band_order[atomicAdd(&d.ctr->band_hist[band_order_key(d, b)], 1)] = b;
+    __syncthreads();
+    for (int b = tid; b < d.n_bands; b += BO_BLOCK) d.band_order[atomicAdd(&pos[band_order_key(d, b)], 1)] = b;
 }
 void launch_band_order(const DeviceBatch& d, cudaStream_t s) {
     if (d.n_bands == 0) return;
-    int grid = (d.n_bands + 255) / 256;
-    grid = grid < 1024 ? grid : 1024;
-    band_hist_kernel<<<grid, 256, 0, s>>>(d);
-    band_scan_kernel<<<1, 1, 0, s>>>(d);
-    band_scatter_kernel<<<grid, 256, 0, s>>>(d);
+    band_order_kernel<<<1, BO_BLOCK, 0, s>>>(d);
 }
 
 // neg_log_posterior (src/parametric.rs:2464-2511) of MetzgerKN at one
-// parameter vector, by one lane: a first FP64 sweep for the rescale's peak
-// (the largest non-upper prediction), a second for the terms in observation
-// order, as the reference sums them.
-__device__ double metzger_nlp_lane(const BandView& b, const double* p) {
-    struct Peak {
-        const uint8_t* up;
-        double mx;
-        __device__ void operator()(int j, double l) {
-            if (!up[j]) mx = fmax(mx, l);
-        }
-    } pk{b.up, -INFINITY};
-    int j_start;
+// parameter vector, by one lane: the terms in observation order, as the
+// reference sums them.
+__device__ double metzger_nlp_lane(MzTables& T, int slot, int col, const BandView& b, const double* p) {
+    MzPeak pk{b.up, -INFINITY};
+    int j_start = b.n;
     double l_peak;
-    bool ok = metzger_sweep64(p, b.t, b.n, pk, j_start, l_peak) && l_peak > 0.0 && isfinite(l_peak);
+    bool ok = mz_sweep(T, p, slot, col, l_peak) && l_peak > 0.0 && isfinite(l_peak);
+    if (ok) mz_visit(T, slot, col, p[3], b.t, b.n, j_start, pk);
     // the predictions before the first visited observation are 0
     double mx = pk.mx / l_peak;
     for (int j = 0; j < (ok ? j_start : b.n); j++)
@@ -592,7 +630,7 @@ __device__ double metzger_nlp_lane(const BandView& b, const double* p) {
     } tm{&b, l_peak, scale, se2, 0.0, 0};
     if (ok) {
         for (int j = 0; j < j_start; j++) tm.term(j, 0.0 * scale);
-        metzger_sweep64(p, b.t, b.n, tm, j_start, l_peak);
+        mz_visit(T, slot, col, p[3], b.t, b.n, j_start, tm);
     } else {
         for (int j = 0; j < b.n; j++) tm.term(j, 0.0 * scale);
     }
@@ -603,48 +641,6 @@ __device__ double metzger_nlp_lane(const BandView& b, const double* p) {
         nlp += 0.5 * dd * dd / (w * w);
     }
     return tm.nll + nlp;
-}
-
-// MetzgerKN's Laplace Hessian as the reference takes it (central differences
-// of the cost, :2623-2693), with the stencil's points spread over the lanes:
-// point 0 is the MAP (its cost f0), points 1 + 4k .. 4 + 4k the four
-// evaluations of the k-th pair (si <= sj).  Warp-collective.
-__device__ void laplace_fd_metzger(const BandView& b, const double* mp, const int* idx, int ns, double* H,
-                                   double& f0) {
-    const int lane = threadIdx.x & 31;
-    const int npts = 1 + 2 * ns * (ns + 1);
-    double c[2] = {0.0, 0.0};
-    for (int r = 0; r < 2; r++) {
-        const int pt = lane + 32 * r;
-        if (pt >= npts) continue;
-        double q[MAXP];
-        for (int t = 0; t < n_params_of(METZGER); t++) q[t] = mp[t];
-        if (pt > 0) {
-            int k = (pt - 1) >> 2, si = 0;
-            while (k >= ns - si) { k -= ns - si; si++; }
-            const int sj = si + k, s4 = (pt - 1) & 3;
-            const int i = idx[si], j = idx[sj];
-            const double hi = 1e-4 * fmax(fabs(mp[i]), 1.0), hj = 1e-4 * fmax(fabs(mp[j]), 1.0);
-            q[i] += (s4 < 2 ? 1.0 : -1.0) * hi;
-            q[j] += ((s4 & 1) == 0 ? 1.0 : -1.0) * hj;
-        }
-        c[r] = metzger_nlp_lane(b, q);
-    }
-    auto cost = [&](int pt) {
-        const double v = pt < 32 ? c[0] : c[1];
-        return __shfl_sync(FULL, v, pt & 31);
-    };
-    f0 = cost(0);
-    int k = 0;
-    for (int si = 0; si < ns; si++) {
-        const double hi = 1e-4 * fmax(fabs(mp[idx[si]]), 1.0);
-        for (int sj = si; sj < ns; sj++, k++) {
-            const double hj = 1e-4 * fmax(fabs(mp[idx[sj]]), 1.0);
-            const double h = (cost(1 + 4 * k) - cost(2 + 4 * k) - cost(3 + 4 * k) + cost(4 + 4 * k)) / (4.0 * hi * hj);
-            H[si * ns + sj] = h;
-            H[sj * ns + si] = h;
-        }
-    }
 }
 
 // Analytic Hessian of neg_log_posterior (src/parametric.rs:2464-2507) over the
@@ -714,13 +710,36 @@ __device__ bool laplace_hessian_analytic(int m, const BandView& b, const double*
     return !__any_sync(FULL, bad);
 }
 
+// sigma from the Hessian's inverse (Jacobi eigen-decomposition, eigenvalue
+// clamp 1e-6), and the band's outputs (:2664-2693); one thread.
+__device__ void laplace_write(BandOut& o, int m, const double* mp, double* H, int ns, double f0) {
+    const int nf = n_params_of(m), se = se_idx_of(m);
+    double ev[MAXP], V[36];
+    jacobi_eigen(H, ns, ev, V);
+    double sls[MAXP];
+    for (int i = 0; i < ns; i++) {
+        double sum = 0.0;
+        for (int k = 0; k < ns; k++) sum += V[i * ns + k] * V[i * ns + k] * (1.0 / fmax(ev[k], 1e-6));
+        sls[i] = 0.5 * log(fmax(sum, 1e-30));
+    }
+    int s2 = 0;
+    for (int i = 0; i < MAXP; i++) {
+        o.mu[i] = i < nf ? mp[i] : NAN;
+        if (i >= nf) o.log_sigma[i] = NAN;
+        else if (i == se) o.log_sigma[i] = log(c_pri_w[m][i]);
+        else o.log_sigma[i] = sls[s2++];
+    }
+    o.elbo = -f0;
+    o.svi_steps = 0;
+}
+
 __global__ void laplace_kernel(DeviceBatch d) {
     int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (warp >= d.n_bands) return;
     warp = d.band_order[warp];
     BandStats bs = d.stats[warp];
     BandOut& o = d.out[warp];
-    if (!bs.valid || o.model < 0) return;
+    if (!bs.valid || o.model < 0 || o.model == METZGER) return;
     BandView b = band_view(d, bs);
     int m = o.model, nf = n_params_of(m), se = se_idx_of(m);
     double* scr = d.scratch64 + 5 * bs.off;
@@ -730,14 +749,10 @@ __global__ void laplace_kernel(DeviceBatch d) {
     for (int i = 0; i < nf; i++)
         if (i != se) idx[ns++] = i;
     double H[36];
-    // the analytic Hessian (forward over the adjoint); MetzgerKN, whose
-    // gradient is itself a finite difference in the reference, and points
-    // with non-finite predictions keep the reference's central differences
-    // (MetzgerKN's with one stencil point per lane)
-    double f0;
-    if (m == METZGER) laplace_fd_metzger(b, mp, idx, ns, H, f0);
-    else f0 = neg_log_posterior_w(m, b, mp, scr);
-    const bool analytic = m == METZGER || (f0 < 1e99 && laplace_hessian_analytic(m, b, mp, idx, ns, H));
+    // the analytic Hessian (forward over the adjoint); points with non-finite
+    // predictions keep the reference's central differences
+    const double f0 = neg_log_posterior_w(m, b, mp, scr);
+    const bool analytic = f0 < 1e99 && laplace_hessian_analytic(m, b, mp, idx, ns, H);
     for (int si = 0; si < ns && !analytic; si++) {
         int i = idx[si];
         double hi = 1e-4 * fmax(fabs(mp[i]), 1.0);
@@ -758,24 +773,78 @@ __global__ void laplace_kernel(DeviceBatch d) {
             H[sj * ns + si] = h;
         }
     }
-    if ((threadIdx.x & 31) == 0) {
-        double ev[MAXP], V[36];
-        jacobi_eigen(H, ns, ev, V);
-        double sls[MAXP];
-        for (int i = 0; i < ns; i++) {
-            double sum = 0.0;
-            for (int k = 0; k < ns; k++) sum += V[i * ns + k] * V[i * ns + k] * (1.0 / fmax(ev[k], 1e-6));
-            sls[i] = 0.5 * log(fmax(sum, 1e-30));
+    if ((threadIdx.x & 31) == 0) laplace_write(o, m, mp, H, ns, f0);
+}
+
+// MetzgerKN, whose gradient is itself a finite difference in the reference,
+// keeps the reference's central differences of the cost (:2623-2693), a block
+// per band with the stencil's points spread over its lanes: point 0 is the MAP
+// (its cost f0), points 1 + 4k .. 4 + 4k the four evaluations of the k-th pair
+// (si <= sj).  The 41 points take 7 values of t0 (metzger_block.cuh).  A basic
+// batch with one MetzgerKN band, GB300: Laplace 6.6 -> 1.9 ms.
+__global__ void __launch_bounds__(MZ_BLOCK) laplace_metzger_kernel(DeviceBatch d) {
+    extern __shared__ __align__(16) unsigned char mz_raw[];
+    MzTables& T = *reinterpret_cast<MzTables*>(mz_raw);
+    __shared__ double s_c[MZ_LANES];
+    constexpr int m = METZGER, np = 5, ns = 4, t0i = 3;  // shape parameters 0 .. 3
+    constexpr int npts = 1 + 2 * ns * (ns + 1);
+    static_assert(npts <= MZ_LANES && n_params_of(m) == np && se_idx_of(m) == ns, "MetzgerKN stencil");
+    const int tid = threadIdx.x;
+    const int n_metzger = d.ctr->band_hist[0];
+    for (int ib = blockIdx.x; ib < n_metzger; ib += gridDim.x) {
+        const int band = d.band_order[ib];
+        const BandStats bs = d.stats[band];
+        BandOut& o = d.out[band];
+        const BandView b = band_view(d, bs);
+        double mp[MAXP];
+        for (int j = 0; j < np; j++) mp[j] = o.pso_params[j];
+        auto step = [&](int i) { return 1e-4 * fmax(fabs(mp[i]), 1.0); };
+        // t0 of table k: 0 the MAP's, 1 and 2 one step up and down, 3 + s4 both
+        // perturbations of the (t0, t0) pair
+        mz_tabulate(T, 7, bs.t_last, [&](int k) {
+            double t0 = mp[t0i];
+            const double h = step(t0i);
+            if (k == 1 || k == 2) t0 += (k == 1 ? 1.0 : -1.0) * h;
+            if (k >= 3) {
+                const int s4 = k - 3;
+                t0 += (s4 < 2 ? 1.0 : -1.0) * h;
+                t0 += ((s4 & 1) == 0 ? 1.0 : -1.0) * h;
+            }
+            return t0;
+        }, tid, MZ_BLOCK);
+        __syncthreads();
+        if (tid < npts) {
+            double q[MAXP];
+            for (int t = 0; t < np; t++) q[t] = mp[t];
+            int slot = 0;
+            if (tid > 0) {
+                int k = (tid - 1) >> 2, si = 0;
+                while (k >= ns - si) { k -= ns - si; si++; }
+                const int sj = si + k, s4 = (tid - 1) & 3;
+                const double hi = step(si), hj = step(sj);
+                q[si] += (s4 < 2 ? 1.0 : -1.0) * hi;
+                q[sj] += ((s4 & 1) == 0 ? 1.0 : -1.0) * hj;
+                if (si == t0i) slot = 3 + s4;
+                else if (sj == t0i) slot = (s4 & 1) == 0 ? 1 : 2;
+            }
+            s_c[tid] = metzger_nlp_lane(T, slot, tid, b, q);
         }
-        int s2 = 0;
-        for (int i = 0; i < MAXP; i++) {
-            o.mu[i] = i < nf ? mp[i] : NAN;
-            if (i >= nf) o.log_sigma[i] = NAN;
-            else if (i == se) o.log_sigma[i] = log(c_pri_w[m][i]);
-            else o.log_sigma[i] = sls[s2++];
+        __syncthreads();
+        if (tid == 0) {
+            double H[36];
+            int k = 0;
+            for (int si = 0; si < ns; si++) {
+                const double hi = step(si);
+                for (int sj = si; sj < ns; sj++, k++) {
+                    const double hj = step(sj);
+                    const double h = (s_c[1 + 4 * k] - s_c[2 + 4 * k] - s_c[3 + 4 * k] + s_c[4 + 4 * k]) / (4.0 * hi * hj);
+                    H[si * ns + sj] = h;
+                    H[sj * ns + si] = h;
+                }
+            }
+            laplace_write(o, m, mp, H, ns, s_c[0]);
         }
-        o.elbo = -f0;
-        o.svi_steps = 0;
+        __syncthreads();
     }
 }
 
@@ -784,8 +853,13 @@ void launch_laplace(const DeviceBatch& d, cudaStream_t s) {
     int64_t threads = (int64_t)d.n_bands * 32;
     laplace_kernel<<<(int)((threads + 127) / 128), 128, 0, s>>>(d);
 }
+void launch_laplace_metzger(const DeviceBatch& d, cudaStream_t s) {
+    if (d.n_bands == 0) return;
+    laplace_metzger_kernel<<<std::min(d.n_bands, d.num_sms), MZ_BLOCK, sizeof(MzTables), s>>>(d);
+}
 
-// profile_t0_refine + profile_refine_all + mag chi2
+// profile_t0_refine + profile_refine_all + mag chi2 of the models other than
+// MetzgerKN, a warp per band: FP32 model evaluation, FP64 terms
 #ifndef LCF_REFINE_BLOCK
 #define LCF_REFINE_BLOCK 128
 #endif
@@ -796,30 +870,21 @@ __global__ void refine_kernel(DeviceBatch d) {
     warp = d.band_order[warp];
     BandStats bs = d.stats[warp];
     BandOut& o = d.out[warp];
-    if (!bs.valid || o.model < 0) return;
+    if (!bs.valid || o.model < 0 || o.model == METZGER) return;
     BandView b = band_view(d, bs);
     int m = o.model, np = n_params_of(m), se = se_idx_of(m), t0i = t0_idx_of(m);
     double* scr = d.scratch64 + 5 * bs.off;
     double mu[MAXP], ls[MAXP];
     for (int j = 0; j < np; j++) { mu[j] = o.mu[j]; ls[j] = o.log_sigma[j]; }
-    // scans of the models other than MetzgerKN: FP32 evaluation, FP64 terms;
-    // MetzgerKN: FP64 sweeps, one scan point per lane
-    const bool fast = m != METZGER;
     const float4* obs = d.obs + bs.off;
-    scan_constants(b, exp(2.0 * mu[se]), scr);
-    if (!fast) {
-        extern __shared__ double rf_keep[];
-        refine_metzger(bs, b, scr, mu, ls, rf_keep + (size_t)(threadIdx.x >> 5) * 32 * MZ_KEEP + lane);
-    }
-    auto scan_ll = [&](const double* p, bool rescale) {
-        return fast ? band_ll_fast(m, p, obs, b, scr) : band_ll_w(m, b, p, scr, rescale);
-    };
+    scan_constants(b, exp(2.0 * mu[se]), scr, lane, 32);
+    __syncwarp();
+    auto scan_ll = [&](const double* p) { return band_ll_fast(m, p, obs, b, scr); };
     // ---- profile_t0_refine
-    if (fast) {
+    {
         double t0_lo = bs.t_first - 30.0, t0_hi = bs.t_peak_all + 5.0;
         if (t0_lo < t0_hi) {
             const int NG = 25;
-            double sx2 = exp(2.0 * mu[se]);
             bool has_b = (m == BAZIN || m == TDE);
             double best_t0 = mu[t0i], best_ll = -INFINITY;
             for (int gi = 0; gi < NG; gi++) {
@@ -831,23 +896,9 @@ __global__ void refine_kernel(DeviceBatch d) {
                 p[0] = 0.0;
                 double saved_b = 0.0;
                 if (has_b) { saved_b = p[1]; p[1] = 0.0; }
-                double sw = 0, sy = 0, sf = 0, syf = 0, sff = 0;
-                if (fast) {
-                    double s5[5];
-                    shape_sums_fast(m, p, obs, b, scr, s5);
-                    sw = s5[0]; sy = s5[1]; sf = s5[2]; syf = s5[3]; sff = s5[4];
-                } else {
-                    metzger_prepare(m, p, b, scr);
-                    Predictor P(m, p, scr);
-                    for (int i = lane; i < b.n; i += 32) {
-                        double sh = P(b, i);
-                        if (b.up[i] || !isfinite(sh)) continue;
-                        double w = 1.0 / (b.var[i] + sx2);
-                        sw += w; sy += w * b.f[i]; sf += w * sh; syf += w * b.f[i] * sh; sff += w * sh * sh;
-                    }
-                    sw = wsum(sw); sy = wsum(sy); sf = wsum(sf); syf = wsum(syf); sff = wsum(sff);
-                    __syncwarp();
-                }
+                double s5[5];
+                shape_sums_fast(m, p, obs, b, scr, s5);
+                const double sw = s5[0], sy = s5[1], sf = s5[2], syf = s5[3], sff = s5[4];
                 if (has_b) {
                     double det = sw * sff - sf * sf;
                     if (fabs(det) > 1e-20) {
@@ -859,7 +910,7 @@ __global__ void refine_kernel(DeviceBatch d) {
                     if (sff > 1e-20 && syf / sff > 1e-10) p[0] = log(syf / sff);
                     else p[0] = saved_la;
                 }
-                double ll = scan_ll(p, true);
+                double ll = scan_ll(p);
                 if (ll > best_ll) { best_ll = ll; best_t0 = t0; }
             }
             double lo1 = best_t0, hi1 = best_t0, thr = best_ll - 0.5;
@@ -869,7 +920,7 @@ __global__ void refine_kernel(DeviceBatch d) {
                 double p[MAXP];
                 for (int j = 0; j < np; j++) p[j] = mu[j];
                 p[t0i] = t0;
-                if (scan_ll(p, false) >= thr) lo1 = t0;
+                if (scan_ll(p) >= thr) lo1 = t0;
                 else break;
             }
             for (int gi = 0; gi < NG; gi++) {
@@ -878,7 +929,7 @@ __global__ void refine_kernel(DeviceBatch d) {
                 double p[MAXP];
                 for (int j = 0; j < np; j++) p[j] = mu[j];
                 p[t0i] = t0;
-                if (scan_ll(p, false) >= thr) hi1 = t0;
+                if (scan_ll(p) >= thr) hi1 = t0;
                 else break;
             }
             mu[t0i] = best_t0;
@@ -886,8 +937,8 @@ __global__ void refine_kernel(DeviceBatch d) {
         }
     }
     // ---- profile_refine_all
-    if (fast) {
-        double map_ll = scan_ll(mu, false);
+    {
+        double map_ll = scan_ll(mu);
         double thr = map_ll - 0.5;
         for (int j = 0; j < np; j++) {
             if (j == se) continue;
@@ -901,7 +952,7 @@ __global__ void refine_kernel(DeviceBatch d) {
                 double p[MAXP];
                 for (int k = 0; k < np; k++) p[k] = mu[k];
                 p[j] = val;
-                double ll = scan_ll(p, false);
+                double ll = scan_ll(p);
                 if (ll >= thr) { l1 = fmin(l1, val); h1 = fmax(h1, val); }
             }
             double prof = fmax((h1 - l1) / 2.0, 1e-6);
@@ -914,7 +965,6 @@ __global__ void refine_kernel(DeviceBatch d) {
     double msum = 0.0;
     int mcount = 0;
     {
-        metzger_prepare(m, mu, b, scr);
         Predictor P(m, mu, scr);
         int npos = 0;
         for (int i = lane; i < b.n; i += 32) npos += (P(b, i) * b.peak > 0.0) ? 1 : 0;
@@ -927,7 +977,6 @@ __global__ void refine_kernel(DeviceBatch d) {
             for (int j = 0; j < np; j++) pso[j] = o.pso_params[j];
             use = pso;
         }
-        metzger_prepare(m, use, b, scr);
         Predictor Q(m, use, scr);
         for (int i = lane; i < b.n; i += 32) {
             double pf = Q(b, i) * b.peak;
@@ -953,8 +1002,19 @@ __global__ void refine_kernel(DeviceBatch d) {
 void launch_refine(const DeviceBatch& d, cudaStream_t s) {
     if (d.n_bands == 0) return;
     int64_t threads = (int64_t)d.n_bands * 32;
-    const size_t smem = (size_t)(LCF_REFINE_BLOCK / 32) * 32 * MZ_KEEP * sizeof(double);
-    refine_kernel<<<(int)((threads + LCF_REFINE_BLOCK - 1) / LCF_REFINE_BLOCK), LCF_REFINE_BLOCK, smem, s>>>(d);
+    refine_kernel<<<(int)((threads + LCF_REFINE_BLOCK - 1) / LCF_REFINE_BLOCK), LCF_REFINE_BLOCK, 0, s>>>(d);
+}
+// The MetzgerKN bands of the refinements: one block per SM (the tables fill
+// its shared memory), the grid draining band_order's MetzgerKN bands.
+void launch_refine_metzger(const DeviceBatch& d, cudaStream_t s) {
+    if (d.n_bands == 0) return;
+    refine_metzger_kernel<<<std::min(d.n_bands, d.num_sms), MZ_BLOCK, sizeof(MzTables), s>>>(d);
+}
+int finalize_init_attributes() {
+    const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaError_t e = cudaFuncSetAttribute(refine_metzger_kernel, a, (int)sizeof(MzTables));
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(laplace_metzger_kernel, a, (int)sizeof(MzTables));
+    return (int)e;
 }
 
 // ---------------------------------------------------------------------------

@@ -183,6 +183,9 @@ struct lcf_ctx {
     cudaStream_t stream_mb = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     int mb_branch = 1;
+    // the MetzgerKN bands' uncertainty and refinements, beside the other bands'
+    cudaStream_t stream_kn = nullptr;
+    cudaEvent_t ev_fork_kn = nullptr, ev_join_kn = nullptr;
     bool mb_timed = false;   // the last enqueued sequence recorded ev[9], ev[10]
     bool mb_branched = false;  // ... and ran MultiBazin on its branch
     std::string err;
@@ -312,6 +315,9 @@ extern "C" int lcf_ctx_create(int device, lcf_ctx** out) {
         cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->ev_done, cudaEventDisableTiming) != cudaSuccess) {
+        cudaStreamCreateWithFlags(&ctx->stream_kn, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&ctx->ev_fork_kn, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&ctx->ev_join_kn, cudaEventDisableTiming) != cudaSuccess ||
         lcf_ctx_destroy(ctx);
         return LCF_E_CUDA;
     }
@@ -337,6 +343,10 @@ extern "C" int lcf_ctx_create(int device, lcf_ctx** out) {
     ctx->pso_rest_per_sm = ctx->cand_bps_rest[0];
     ctx->lb_grid = lbfgs_grid(ctx->num_sms);
     // RNG tables
+    if (finalize_init_attributes() != 0) {
+        lcf_ctx_destroy(ctx);
+        return LCF_E_CUDA;
+    }
     std::vector<float> draws((size_t)3 * DRAWS_PER_SEED);
     // the SVI noise, then Adam's bias corrections 1 / (1 - 0.9^t) and
     // 1 / (1 - 0.999^t) for t = 1 .. SVI_STEPS (the powers by the repeated FP64
@@ -399,6 +409,9 @@ extern "C" void lcf_ctx_destroy(lcf_ctx* ctx) {
     if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
     if (ctx->ev_join) cudaEventDestroy(ctx->ev_join);
     if (ctx->stream_mb) cudaStreamDestroy(ctx->stream_mb);
+    if (ctx->ev_fork_kn) cudaEventDestroy(ctx->ev_fork_kn);
+    if (ctx->ev_join_kn) cudaEventDestroy(ctx->ev_join_kn);
+    if (ctx->stream_kn) cudaStreamDestroy(ctx->stream_kn);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
 }
@@ -806,6 +819,24 @@ static void enqueue_pipeline(lcf_ctx* ctx) {
     stage_event(ctx, ctx->ev[0], s);
     cudaMemsetAsync(ctx->res.p, 0xff, (size_t)std::max(ctx->n_bands, 1) * 44 * sizeof(PsoResult), s);
     cudaMemsetAsync(ctx->ctr.p, 0, sizeof(Counters), s);
+// The MetzgerKN bands' uncertainty (unless it was given) and refinements on
+// their own stream: a few bands whose chains of ODE steps are far longer than
+// the other models' run beside those instead of before them.  The caller joins
+// ev_join_kn.  Returns the launches.
+static int enqueue_metzger(lcf_ctx* ctx, bool uncertainty) {
+    const DeviceBatch& d = ctx->db;
+    cudaStream_t q = ctx->stream_kn;
+    cudaEventRecord(ctx->ev_fork_kn, ctx->stream);
+    cudaStreamWaitEvent(q, ctx->ev_fork_kn, 0);
+    if (uncertainty) {
+        if (ctx->opts.method == LCF_METHOD_SVI) launch_svi_metzger(d, q);
+        else launch_laplace_metzger(d, q);
+    }
+    launch_refine_metzger(d, q);
+    cudaEventRecord(ctx->ev_join_kn, q);
+    return uncertainty ? 2 : 1;
+}
+
     cudaMemsetAsync(ctx->fits.p, 0xff, (size_t)std::max(ctx->n_bands, 1) * 8 * sizeof(ModelFit), s);
     launch_prep(d, s); L++;
     stage_event(ctx, ctx->ev[1], s);
@@ -860,7 +891,8 @@ static void enqueue_pipeline(lcf_ctx* ctx) {
         launch_t0_pick(d, 3, 1, s); L++;
     }
     stage_event(ctx, ctx->ev[4], s);
-    launch_band_order(d, s); L += 3;
+    launch_band_order(d, s); L++;
+    L += enqueue_metzger(ctx, true);
     if (o.method == LCF_METHOD_SVI) launch_svi(d, s);
     else launch_laplace(d, s);
     L++;
@@ -877,6 +909,7 @@ static int run_pipeline(lcf_ctx* ctx) {
     cudaGetLastError();  // a failed query elsewhere in the process must not be reported as ours
     // set per fit (a graph replay does not run enqueue_pipeline)
     ctx->mb_timed = ctx->opts.run_multi_bazin != 0;
+    cudaStreamWaitEvent(s, ctx->ev_join_kn, 0);
     ctx->mb_branched = ctx->mb_timed && ctx->mb_branch != 0;
     uint64_t gkey = ctx->layout_key ^ ((uint64_t)(uintptr_t)ctx->db.times * 31) ^ ((uint64_t)ctx->n_obs << 7) ^
                     ((uint64_t)(ctx->cfg + 1) << 56) ^ ((uint64_t)(ctx->mb_branch + 1) << 52);
@@ -1219,7 +1252,7 @@ static void enqueue_finalize(lcf_ctx* ctx, bool given, size_t sel_bytes) {
     cudaEventRecord(ctx->ev[2], s);
     cudaEventRecord(ctx->ev[3], s);
     cudaEventRecord(ctx->ev[8], s);
-    launch_band_order(d, s); L += 3;
+    launch_band_order(d, s); L++;
     cudaEventRecord(ctx->ev[4], s);
     if (!given) {
         if (ctx->opts.method == LCF_METHOD_SVI) launch_svi(d, s);
@@ -1232,6 +1265,7 @@ static void enqueue_finalize(lcf_ctx* ctx, bool given, size_t sel_bytes) {
     cudaEventRecord(ctx->ev[7], s);
     ctx->launches = L;
 }
+    L += enqueue_metzger(ctx, !given);
 
 extern "C" int lcf_finalize_batch(lcf_ctx* ctx, const lcf_bands_csr* in, const lcf_pso_selection* sel, int method,
                                   lcf_fit_outputs* out) {
@@ -1239,6 +1273,7 @@ extern "C" int lcf_finalize_batch(lcf_ctx* ctx, const lcf_bands_csr* in, const l
     if (int rc = busy(ctx)) return rc;
     if (!in || !sel || !out) return set_err(ctx, LCF_E_INVALID, "null argument");
     const bool given = sel->svi_mu != nullptr || sel->svi_log_sigma != nullptr;
+    cudaStreamWaitEvent(s, ctx->ev_join_kn, 0);
     if (given && !(sel->svi_mu && sel->svi_log_sigma))
         return set_err(ctx, LCF_E_INVALID, "svi_mu and svi_log_sigma are given together");
     if (!given && method != LCF_METHOD_SVI && method != LCF_METHOD_LAPLACE)

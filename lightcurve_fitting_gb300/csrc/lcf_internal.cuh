@@ -225,7 +225,7 @@ struct Counters {
     unsigned long long lb_obs_evals_by_model[8];  // observation x (cost + gradient) evaluations, by model
     unsigned long long lb_fp64_obs_evals_by_model[8];  // of which in FP64 (ff range fallback)
     int32_t sort_hist[8][256];  // per slot: key histogram, then offsets, of the device task sort
-    int32_t band_hist[16];      // bands by selected model: histogram, then offsets (band_order)
+    int32_t band_hist[16];      // bands by selected model, in band_order's grouping (0: MetzgerKN)
     int32_t polish_hist[256];   // bands by length: histogram, then offsets (polish_order)
     int32_t lb_next[8];         // per model: next index of the polish queue (eight lanes a band)
     int32_t lb_next_long[8];    // per model: next index of its long bands (a warp a band)
@@ -357,7 +357,7 @@ int launch_joint(const DeviceBatch& d, cudaStream_t s);
 size_t joint_smem_bytes(int max_obs, int max_d);
 // finalize.cu
 void launch_laplace(const DeviceBatch& d, cudaStream_t s);
-// bands grouped by selected model into d.band_order (three launches)
+// bands grouped by selected model into d.band_order, their counts into ctr->band_hist
 void launch_band_order(const DeviceBatch& d, cudaStream_t s);
 void launch_refine(const DeviceBatch& d, cudaStream_t s);
 double probe_fp32_tflops(int num_sms);
@@ -368,6 +368,12 @@ int probe_fp64_peaks(int num_sms, double* out9);
 int probe_ff(int num_sms, double* out80);
 double probe_mufu_gops(int num_sms);
 void launch_band_cost(int model, const float4* obs, int n, float t_last, const double* params, int n_eval,
+// the MetzgerKN bands of SVI, Laplace and the refinements, which the kernels
+// above leave out (after launch_band_order)
+void launch_svi_metzger(const DeviceBatch& d, cudaStream_t s);
+void launch_laplace_metzger(const DeviceBatch& d, cudaStream_t s);
+void launch_refine_metzger(const DeviceBatch& d, cudaStream_t s);
+int finalize_init_attributes();
                       int with_prior, double* costs, float* scratch, cudaStream_t s);
 
 // Host-side generation of the RNG tables (host.cpp)

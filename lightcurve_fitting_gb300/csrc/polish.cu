@@ -18,6 +18,8 @@
 // stored.  Adam runs in FP64 with one variational parameter per lane.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "grads_f32.cuh"
 #include "lane_cost.cuh"
 #include "lbfgs_group.cuh"
@@ -86,8 +88,6 @@ int lbfgs_grid(int num_sms) {
     return num_sms * n;
 }
 
-void launch_lbfgs(const DeviceBatch& d, int model_mask, cudaStream_t s) {
-    if (d.n_bands == 0) return;
 // A batch of fewer bands than five per warp of the grid waits for its longest
 // polishes: every band then gets a warp, and the SMs start at staggered models
 // so that the models' queues drain together.  Larger batches are bound by
@@ -104,6 +104,8 @@ int polish_warp_obs(int n_bands, int lb_grid) {
     return polish_small(n_bands, lb_grid) ? 0 : 96;
 }
 
+void launch_lbfgs(const DeviceBatch& d, int model_mask, cudaStream_t s) {
+    if (d.n_bands == 0) return;
     // The bands of LB_LONG_OBS observations or more are summed in the order of
     // 32 lanes, the others in that of eight, whatever the batch and however
     // many lanes evaluate them: a band's fit is the same in any batch.
@@ -565,6 +567,33 @@ struct SviDeferred {
     int floored;  // a deferred upper limit hit the CDF floor (warp-uniform)
 };
 
+// Sums of seven values over the lanes in `act`, in lane order: lane l returns
+// the sum of value l & 7 (0 for 7).  Through shared memory, one load and one
+// FP64 addition a lane in `act`; broadcasting every lane's seven values took
+// 14 shuffles each, which set the time of a step whose upper limits are at the
+// floor across the band.  Blocks of four warps.
+static __device__ __noinline__ double ordered_lane_sum(double d0, double d1, double d2, double d3, double d4,
+                                                       double d5, double d6, unsigned act) {
+    __shared__ double buf[4][7][33];
+    const int lane = threadIdx.x & 31, c = lane & 7;
+    double(*mine)[33] = buf[(threadIdx.x >> 5) & 3];
+    if ((act >> lane) & 1) {
+        mine[0][lane] = d0;
+        mine[1][lane] = d1;
+        mine[2][lane] = d2;
+        mine[3][lane] = d3;
+        mine[4][lane] = d4;
+        mine[5][lane] = d5;
+        mine[6][lane] = d6;
+    }
+    __syncwarp();
+    double r = 0.0;
+    if (c < 7)
+        for (unsigned m = act; m; m &= m - 1) r += mine[c][__ffs(m) - 1];
+    __syncwarp();
+    return r;
+}
+
 // The reference's gradient terms of the upper limits that upper_ratio_f32
 // deferred: those whose quantised CDF 0.5 (1 + erf) holds fewer than 64 units
 // of 2^-53 (src/parametric.rs:2336-2352: dpred = -phi / (cdf sigma) times each
@@ -681,23 +710,8 @@ __device__ __noinline__ SviDeferred svi_deferred_pass(const float4* obs, const f
             dx[se] += (phi / cdf) * (-(uf - pd) * sxx / (sd * tvd));
         }
     }
-    // warp totals: only the lanes that deferred something contribute (few),
-    // so each of those lanes' components is broadcast and lane l keeps
-    // component l & 7
     SviDeferred r;
-    r.dlx = 0.0;
-    unsigned act = __ballot_sync(FULL, any);
-    while (act) {
-        const int src = __ffs(act) - 1;
-        act &= act - 1;
-        double mine = 0.0;
-#pragma unroll
-        for (int q = 0; q < np; q++) {
-            const double v = __shfl_sync(FULL, dx[q], src);
-            if (q == (lane & 7)) mine = v;
-        }
-        r.dlx += mine;
-    }
+    r.dlx = ordered_lane_sum(dx[0], dx[1], dx[2], dx[3], dx[4], dx[5], dx[6], __ballot_sync(FULL, any));
     r.floored = warp_or(floored);
     return r;
 }
@@ -815,9 +829,29 @@ __device__ __forceinline__ bool svi_sample_loglik(const float4* obs, int n, cons
     return true;
 }
 
-template <int M>
-__device__ void svi_band(const DeviceBatch& d, int b) {
-    const int lane = threadIdx.x & 31, j = lane & 7;
+// A band's SVI by W warps (1 or SVI_SAMPLES): warp w evaluates samples w,
+// w + W, ... of every step; warp 0 then adds the samples' terms in the
+// reference's order and takes the Adam step.  The warps share the variational
+// parameters and the samples' gradients in shared memory.
+struct SviShared {
+    double vp[16];                   // mu, then log sigma
+    double df[SVI_SAMPLES][8];       // per sample: d (log-likelihood + prior) / d theta_j
+    double dfs[SVI_SAMPLES][8];      // the same times sigma_j
+    double eps[SVI_SAMPLES][8];
+    double e[SVI_SAMPLES];           // log-likelihood + prior
+    int ok[SVI_SAMPLES];             // 0: the reference skips the sample
+    int stop;
+};
+
+template <int W>
+__device__ __forceinline__ void svi_sync() {
+    if constexpr (W == 1) __syncwarp();
+    else __syncthreads();
+}
+
+template <int M, int W>
+__device__ void svi_band(const DeviceBatch& d, int b, SviShared& sh, MzWarp* mz = nullptr) {
+    const int lane = threadIdx.x & 31, w = W == 1 ? 0 : threadIdx.x >> 5, j = lane & 7;
     const BandStats bs = d.stats[b];
     BandOut& o = d.out[b];
     if (!bs.valid || o.model != M) return;
@@ -833,93 +867,76 @@ __device__ void svi_band(const DeviceBatch& d, int b) {
     // 1 / variance, formed once: the FP64 divisions of the step are its
     // costliest instructions on this part (a few are left: sqrt, Adam's step)
     const double ipw2_j = own ? 1.0 / pw2_j : 0.0;
-    // lane i < 2 np owns variational parameter i (mu_i, then log sigma_i)
+    // warp 0, lane i < 2 np owns variational parameter i (mu_i, then log sigma_i)
     double vp = 0.0, am = 0.0, av = 0.0;
     if (lane < np) vp = o.pso_params[lane];
     else if (lane < 2 * np) vp = -1.0;
+    if (w == 0 && lane < 16) sh.vp[lane] = vp;
     const double* eps_tab = d.svi_eps + (size_t)(np - 5) * SVI_STEPS * SVI_SAMPLES * 7;
     const double ln_2pie = 2.8378770664093453;  // ln(2 pi e)
     double ema = -INFINITY, best_ema = -INFINITY, final_elbo = -INFINITY;
     int no_imp = 0, steps = 0;
-    // MetzgerKN: per step, lanes 0..15 sweep samples 0..3 (value + 4 derivatives per observation)
-    float* mscr = d.scratch_svi + 20 * bs.off;
+    float* mscr = d.scratch_svi + 20 * bs.off;  // MetzgerKN: a sample's value + 4 derivatives per observation
     struct ObsTimes {
         const float4* o;
         __device__ float operator()(int q) const { return o[q].x + o[q].y; }
     } otimes{obs};
     for (int step = 0; step < SVI_STEPS; step++) {
+        svi_sync<W>();  // the parameters of this step (or the end) are written
+        if (step > 0 && sh.stop) break;
         steps = step + 1;
-        const double mu_j = __shfl_sync(FULL, vp, j);
-        const double ls_j = __shfl_sync(FULL, vp, (np + j) & 31);
+        const double mu_j = own ? sh.vp[j] : 0.0;
+        const double ls_j = own ? sh.vp[np + j] : 0.0;
         // sigma = e^(log sigma) in double-float on the FP32 pipe (log sigma is
         // clamped to [-6, 2]; ~1e-14 relative): the FP64 exp was the step's
         // costliest remaining FP64 call
         const double sg_j = own ? ff_to(ff_exp(ff_from(ls_j))) : 0.0;
-        if constexpr (M == METZGER) {
-            double mu[MAXP], sg[MAXP];
-#pragma unroll
-            for (int q = 0; q < np; q++) { mu[q] = __shfl_sync(FULL, mu_j, q); sg[q] = __shfl_sync(FULL, sg_j, q); }
-            // lane 4 s + k sweeps sample s with the tangent of parameter k
-            // only (the four-tangent sweep's arithmetic, split over lanes)
-            const int smp = lane >> 2, tan = lane & 3;
-            bool mz_ok = false;
-            float mz_lp = 0.0f, mz_lpd = 0.0f;
-            if (lane < 4 * SVI_SAMPLES) {
-                const double* ep = eps_tab + ((size_t)step * SVI_SAMPLES + smp) * 7;
-                float pv[MAXP];
-                for (int q = 0; q < np; q++) pv[q] = (float)(mu[q] + sg[q] * ep[q]);
-                mz_ok = metzger_dual_raw<1>(pv, tan, (float)bs.t_last, otimes, n, mscr + (size_t)smp * 5 * n, mz_lp,
-                                            &mz_lpd);
-            }
-            __syncwarp();
-            // normalise by the peak (its tangent included): each lane its
-            // tangent column, then the value column
-            if (lane < 4 * SVI_SAMPLES) {
-                float* ms = mscr + (size_t)smp * 5 * n;
-                const float ip = 1.0f / mz_lp;
-                for (int q = 0; q < n; q++) {
-                    const float y = ms[q * 5] * ip;
-                    ms[q * 5 + 1 + tan] = mz_ok ? (ms[q * 5 + 1 + tan] - y * mz_lpd) * ip : 0.0f;
-                }
-            }
-            __syncwarp();
-            if (lane < 4 * SVI_SAMPLES && tan == 0) {
-                float* ms = mscr + (size_t)smp * 5 * n;
-                const float ip = 1.0f / mz_lp;
-                for (int q = 0; q < n; q++) ms[q * 5] = mz_ok ? ms[q * 5] * ip : 0.0f;
-            }
-            __syncwarp();
-        }
-        double gmu_j = 0.0, gls_j = 0.0, elbo_sum = 0.0;
-        for (int k = 0; k < SVI_SAMPLES; k++) {
+        for (int k = w; k < SVI_SAMPLES; k += W) {
             const double* ep = eps_tab + ((size_t)step * SVI_SAMPLES + k) * 7;
             const double eps_j = own ? ep[j] : 0.0;
             const double th_j = mu_j + sg_j * eps_j;
             float pf[MAXP];
 #pragma unroll
             for (int q = 0; q < MAXP; q++) pf[q] = q < np ? __shfl_sync(FULL, (float)th_j, q) : 0.0f;
+            if constexpr (M == METZGER)
+                metzger_dual_warp(mz[w], pf, (float)bs.t_last, otimes, n, mscr + (size_t)k * 5 * n);
             double lls, dlx;
             float dl_tot;
             int floored;
-            if (!svi_sample_loglik<M>(obs, n, pf, th_j, mscr + (size_t)k * 5 * n, lls, dl_tot, dlx, floored))
-                continue;
-            // lane j: total d loglik / d theta_j (FP32 terms, plus the FP64
-            // terms of deferred upper limits), then its prior and ELBO terms
-            const double dl_j = (double)__shfl_sync(FULL, dl_tot, (4 * j) & 31) + dlx;
-            double lp_j = 0.0;
-            if (own) {
-                const double dd = th_j - pc_j;
-                const double dq = dd * ipw2_j;
-                lp_j = -0.5 * dd * dq;
-                const double df = dl_j - dq;
-                gmu_j += df;
-                gls_j += df * sg_j * eps_j;
+            const bool ok = svi_sample_loglik<M>(obs, n, pf, th_j, mscr + (size_t)k * 5 * n, lls, dl_tot, dlx, floored);
+            if (ok) {
+                // lane j: total d loglik / d theta_j (FP32 terms, plus the FP64
+                // terms of deferred upper limits), then its prior and ELBO terms
+                const double dl_j = (double)__shfl_sync(FULL, dl_tot, (4 * j) & 31) + dlx;
+                double lp_j = 0.0, df = 0.0;
+                if (own) {
+                    const double dd = th_j - pc_j;
+                    const double dq = dd * ipw2_j;
+                    lp_j = -0.5 * dd * dq;
+                    df = dl_j - dq;
+                }
+                const double lp = dot8(lp_j, 1.0);
+                if (lane < 8) {
+                    sh.df[k][j] = df;
+                    sh.dfs[k][j] = df * sg_j;
+                    sh.eps[k][j] = eps_j;
+                }
+                if (lane == 0) sh.e[k] = lls + lp;
             }
-            const double lp = dot8(lp_j, 1.0);
-            elbo_sum += lls + lp;
+            if (lane == 0) sh.ok[k] = ok;
+        }
+        svi_sync<W>();
+        if (w != 0) continue;
+        double gmu_j = 0.0, gls_j = 0.0, elbo_sum = 0.0;
+#pragma unroll
+        for (int q = 0; q < SVI_SAMPLES; q++) {
+            if (!sh.ok[q]) continue;
+            gmu_j += sh.df[q][j];
+            gls_j += sh.dfs[q][j] * sh.eps[q][j];
+            elbo_sum += sh.e[q];
         }
         const double ns = (double)SVI_SAMPLES;
-        const double ent = dot8(own ? ls_j : 0.0, 1.0) + 0.5 * (double)np * ln_2pie;
+        const double ent = dot8(ls_j, 1.0) + 0.5 * (double)np * ln_2pie;
         final_elbo = elbo_sum / ns + ent;
         // Adam, lane i owns variational parameter i
         const double gmu_i = __shfl_sync(FULL, gmu_j, lane & 7);
@@ -936,15 +953,18 @@ __device__ void svi_band(const DeviceBatch& d, int b) {
             vp -= SVI_LR * mh / (sqrt(vh) + 1e-8);
         }
         if (lane >= np && lane < 2 * np) vp = fmin(fmax(vp, -6.0), 2.0);
+        bool stop = false;
         if (step >= 200) {
             if (ema == -INFINITY) ema = final_elbo;
             else ema = 0.1 * final_elbo + 0.9 * ema;
             bool imp = ema - best_ema > 0.01 * fmax(fabs(best_ema), 1e-10);
             if (imp) { best_ema = ema; no_imp = 0; }
-            else if (++no_imp >= 50) break;
+            else if (++no_imp >= 50) stop = true;
         }
-        __syncwarp();  // MetzgerKN scratch rows are rewritten next step
+        if (lane < 16) sh.vp[lane] = vp;
+        if (lane == 0) sh.stop = stop;
     }
+    if (w != 0) return;
     const double ln4 = 1.3862943611198906;
     double out_v = lane < np ? vp : vp + ln4;
     if (lane < np) o.mu[lane] = out_v;
@@ -957,34 +977,52 @@ __device__ void svi_band(const DeviceBatch& d, int b) {
     }
 }
 
-// One warp per band, in band_order (grouped by selected model, so that the
-// warps of a model run together and share its code).
-#ifndef LCF_SVI_BLOCK
-#define LCF_SVI_BLOCK 128
-#endif
-__global__ void __launch_bounds__(LCF_SVI_BLOCK) svi_kernel(DeviceBatch d) {
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (warp >= d.n_bands) return;
-    const int b = d.band_order[warp];
-    const int m = d.out[b].model;
-    if (m < 0) return;
-    switch (m) {
-        case BAZIN: svi_band<BAZIN>(d, b); break;
-        case VILLAR: svi_band<VILLAR>(d, b); break;
-        case TDE: svi_band<TDE>(d, b); break;
-        case ARNETT: svi_band<ARNETT>(d, b); break;
-        case MAGNETAR: svi_band<MAGNETAR>(d, b); break;
-        case SHOCK: svi_band<SHOCK>(d, b); break;
-        case AFTERGLOW: svi_band<AFTERGLOW>(d, b); break;
-        default: svi_band<METZGER>(d, b); break;
+// The bands in band_order (grouped by selected model, so that the warps
+// resident on an SM share one model's code) past the MetzgerKN ones, W warps a
+// band.
+constexpr int SVI_BLOCK = 32 * SVI_SAMPLES;
+template <int W>
+__global__ void __launch_bounds__(SVI_BLOCK, 3) svi_kernel(DeviceBatch d) {
+    __shared__ SviShared shared[SVI_SAMPLES / W];
+    const int k = threadIdx.x / (32 * W), i = d.ctr->band_hist[0] + blockIdx.x * (SVI_SAMPLES / W) + k;
+    if (i >= d.n_bands) return;
+    SviShared& sh = shared[k];
+    const int b = d.band_order[i];
+    switch (d.out[b].model) {
+        case BAZIN: svi_band<BAZIN, W>(d, b, sh); break;
+        case VILLAR: svi_band<VILLAR, W>(d, b, sh); break;
+        case TDE: svi_band<TDE, W>(d, b, sh); break;
+        case ARNETT: svi_band<ARNETT, W>(d, b, sh); break;
+        case MAGNETAR: svi_band<MAGNETAR, W>(d, b, sh); break;
+        case SHOCK: svi_band<SHOCK, W>(d, b, sh); break;
+        case AFTERGLOW: svi_band<AFTERGLOW, W>(d, b, sh); break;
+        default: break;
+    }
+}
+// The MetzgerKN bands (band_order's first), four warps a
+// band, the grid draining them.
+__global__ void __launch_bounds__(SVI_BLOCK) svi_metzger_kernel(DeviceBatch d) {
+    __shared__ SviShared sh;
+    __shared__ MzWarp mz[SVI_SAMPLES];
+    const int n_metzger = d.ctr->band_hist[0];
+    for (int i = blockIdx.x; i < n_metzger; i += gridDim.x) {
+        svi_band<METZGER, SVI_SAMPLES>(d, d.band_order[i], sh, mz);
+        __syncthreads();
     }
 }
 
+// The 1000-step chain bounds a batch that does not keep the chip's warp slots
+// filled: four warps a band then shorten it (1,000 uneven sources with a warp
+// / four warps a band: 62 / 42 ms, one source 3.2 / 1.7).  A larger batch is
+// bound by throughput and runs a warp a band (10,000 sources: 175 / 203 ms).
 void launch_svi(const DeviceBatch& d, cudaStream_t s) {
     if (d.n_bands == 0) return;
-    int block = LCF_SVI_BLOCK;
-    int64_t threads = (int64_t)d.n_bands * 32;
-    svi_kernel<<<(int)((threads + block - 1) / block), block, 0, s>>>(d);
+    if (d.n_bands <= 4096) svi_kernel<SVI_SAMPLES><<<d.n_bands, SVI_BLOCK, 0, s>>>(d);
+    else svi_kernel<1><<<(d.n_bands + SVI_SAMPLES - 1) / SVI_SAMPLES, SVI_BLOCK, 0, s>>>(d);
+}
+void launch_svi_metzger(const DeviceBatch& d, cudaStream_t s) {
+    if (d.n_bands == 0) return;
+    svi_metzger_kernel<<<std::min(d.n_bands, 5 * d.num_sms), SVI_BLOCK, 0, s>>>(d);
 }
 
 // ---------------------------------------------------------------------------
