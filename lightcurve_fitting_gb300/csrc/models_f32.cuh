@@ -128,6 +128,19 @@ struct VillarF {
         float c3 = fmaxf(beta * tf - 1.0f + beta * gamma, 0.0f);
         return c1 + c2 + c3;
     }
+    // The same in the swarms' fast arithmetic, each rounding spelled out: the
+    // one-warp and the block-run swarms have to order infeasible particles
+    // alike, and the compiler contracts the plain form by its surroundings.
+    __device__ static float constraint_swarm(const float* p) {
+        const float beta = p[1], gamma = expf(p[2]), tr = expf(p[4]), tf = expf(p[5]);
+        float rtr;
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rtr) : "f"(tr));
+        const float bg = __fmul_rn(beta, gamma);
+        const float c1 = fmaxf(__fadd_rn(bg, -1.0f), 0.0f);
+        const float c2 = fmaxf(__fmaf_rn(expf(__fmul_rn(-gamma, rtr)), __fmaf_rn(tf, rtr, -1.0f), -1.0f), 0.0f);
+        const float c3 = fmaxf(__fadd_rn(__fmaf_rn(beta, tf, -1.0f), bg), 0.0f);
+        return __fadd_rn(__fadd_rn(c1, c2), c3);
+    }
 };
 
 struct TdeF {
@@ -300,6 +313,33 @@ struct Nll {
         } else {
             nonfinite = 1;
         }
+    }
+    // The same with the terms outside FP32's squares out of line, for loops
+    // that are bound by instruction fetch (those terms take a third of the
+    // code).  Loops that fit the instruction cache keep obs(): the call's
+    // registers cost them more.
+    __device__ __forceinline__ void obs_outlined(const float4& o, float pred, int st, float se2) {
+        float term;
+        if (st == ST_OK && ordinary(o, pred, se2, term)) add(term);
+        else *this = obs_call(*this, o, pred, st, se2);
+    }
+    // The term of an observation whose square FP32 holds; false for another.
+    static __device__ __forceinline__ bool ordinary(const float4& o, float pred, float se2, float& term) {
+        const float tv = fabsf(o.w) + se2, is = rsqrtf(tv);
+        if (o.w < 0.0f) {
+            const float z = (o.z - pred) * is;
+            if (!(z > -1e15f)) return false;
+            term = -log_normal_cdf_f(z);
+        } else {
+            const float r = (pred - o.z) * is;
+            if (!(fabsf(r) < 1e15f)) return false;
+            term = r * r + logf(tv);
+        }
+        return true;
+    }
+    static __device__ __noinline__ Nll obs_call(Nll a, float4 o, float pred, int st, float se2) {
+        a.obs(o, pred, st, se2);
+        return a;
     }
     // cost = (sum + prior / n) / n in FP64 (inv_n = 1 / n: the FP64 pipe runs
     // at 1/64 of the FP32 rate, and two divisions per evaluation would cost as

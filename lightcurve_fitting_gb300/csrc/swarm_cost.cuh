@@ -27,44 +27,46 @@ struct TaskCtx {
 };
 
 // Negative log-likelihood terms of observations i0, i0 + stride, ... < n.
+// Not unrolled: the swarms of several models share an SM's instruction caches,
+// and the model-selection launch lost 10.6 cycles an issued instruction to
+// fetch.  One observation in the loop, its rare terms out of line: model
+// selection 423 -> 388 ms at 10,000 uneven sources and 70 -> 55 ms at 1,000,
+// the t0 search 106 -> 86 and 46 -> 31 ms.
 template <class M>
 __device__ __forceinline__ Nll nll_loop(const M& m, const float4* obs, int n, float se2, int i0 = 0, int stride = 1) {
     Nll acc;
     acc.reset();
-#pragma unroll 2
+#pragma unroll 1
     for (int i = i0; i < n; i += stride) {
         float4 o = obs[i];
         int st = ST_OK;
         float pr = m.eval(o.x, o.y, st);
-        acc.obs(o, pr, st, se2);
+        acc.obs_outlined(o, pr, st, se2);
     }
     return acc;
 }
 
 // MultiBazin prediction: sum of K Bazin components + B (src/parametric.rs:932-940)
 template <int K>
-__device__ __forceinline__ Nll nll_multibazin(const float* p, const float4* obs, int n, float se2, int i0 = 0,
-                                              int stride = 1) {
-    float la[K], t0[K], itr[K], itf[K], dif[K];
+struct MultiBazinF {
+    float la[K], t0[K], itr[K], itf[K], dif[K], B;
+    __device__ __forceinline__ void init(const float* p) {
 #pragma unroll
-    for (int c = 0; c < K; c++) {
-        la[c] = p[4 * c];
-        t0[c] = p[4 * c + 1];
-        itr[c] = expf(-p[4 * c + 2]);
-        itf[c] = expf(-p[4 * c + 3]);
-        dif[c] = itr[c] * expm1f(p[4 * c + 2] - p[4 * c + 3]);
+        for (int c = 0; c < K; c++) {
+            la[c] = p[4 * c];
+            t0[c] = p[4 * c + 1];
+            itr[c] = expf(-p[4 * c + 2]);
+            itf[c] = expf(-p[4 * c + 3]);
+            dif[c] = itr[c] * expm1f(p[4 * c + 2] - p[4 * c + 3]);
+        }
+        B = p[4 * K];
     }
-    float B = p[4 * K];
-    Nll acc;
-    acc.reset();
-    for (int i = i0; i < n; i += stride) {
-        float4 o = obs[i];
+    __device__ __forceinline__ float eval(float th, float tl, int& st) const {
         float sum = 0.0f, bigL = -INFINITY;
-        int st = ST_OK;
 #pragma unroll
         for (int c = 0; c < K; c++) {
             // one Bazin component in log space (as BazinF::eval)
-            float dt = (o.x - t0[c]) + o.y;
+            float dt = (th - t0[c]) + tl;
             float xf = -dt * itf[c], xr = -dt * itr[c];
             if (xf > 80.0f) {
                 if (xf > LN_DBL_MAX || la[c] + xf > LN_DBL_MAX) { st = ST_NONFINITE; continue; }
@@ -74,15 +76,84 @@ __device__ __forceinline__ Nll nll_multibazin(const float* p, const float4* obs,
             if (L > BIG_L) bigL = fmaxf(bigL, L) + log1pf(expf(-fabsf(bigL - L)));
             else sum += expf(L);
         }
-        float pr = 0.0f;
         if (st == ST_OK && bigL > -INFINITY) {
             // FP64 sum overflows to +inf past ln DBL_MAX: non-finite prediction
-            if (bigL > LN_DBL_MAX) st = ST_NONFINITE;
-            else { st = ST_BIG; pr = bigL; }
-        } else {
-            pr = sum + B;
+            if (bigL > LN_DBL_MAX) { st = ST_NONFINITE; return 0.0f; }
+            st = ST_BIG;
+            return bigL;
         }
+        return sum + B;
+    }
+};
+template <int K>
+__device__ __forceinline__ Nll nll_multibazin(const float* p, const float4* obs, int n, float se2, int i0 = 0,
+                                              int stride = 1) {
+    MultiBazinF<K> e;
+    e.init(p);
+    Nll acc;
+    acc.reset();
+    for (int i = i0; i < n; i += stride) {
+        float4 o = obs[i];
+        int st = ST_OK;
+        float pr = e.eval(o.x, o.y, st);
         acc.obs(o, pr, st, se2);
+    }
+    return acc;
+}
+
+// ---------------------------------------------------------------------------
+// A swarm run by a whole block (pso.cu): warp 0 keeps the swarm, and every
+// evaluation round is spread over the block's warps.  The particles' positions
+// and the terms pass through shared memory; warp 0 adds the terms in the
+// observations' order, so the costs are those of a warp on its own.
+// ---------------------------------------------------------------------------
+constexpr int TEAM_ROWS = 128;  // observations (of each lane's share) whose terms are held at once
+struct SwarmTeam {
+    float* pos;    // [parameter][lane]
+    float* terms;  // [TEAM_ROWS][lane]
+    int warp, n_warps;
+};
+
+// Lane (u, s)'s terms of observations u, u + s, ... < n (n = 0: none), over a
+// band of n_band observations.  Block-collective; warp 0 returns the sums.
+template <class M>
+__device__ __forceinline__ Nll nll_team(const M& m, const float4* obs, int n, int n_band, float se2, int u, int s,
+                                        const SwarmTeam& tm) {
+    Nll acc;
+    acc.reset();
+    const int lane = threadIdx.x & 31;
+    const int rows = (n_band + s - 1) / s;
+    for (int c0 = 0; c0 < rows; c0 += TEAM_ROWS) {
+        const int c1 = min(rows, c0 + TEAM_ROWS);
+        if (c0) __syncthreads();
+#pragma unroll 1
+        for (int r = c0 + tm.warp; r < c1; r += tm.n_warps) {
+            const int i = u + r * s;
+            if (i >= n) continue;
+            const float4 o = obs[i];
+            int st = ST_OK;
+            const float pr = m.eval(o.x, o.y, st);
+            float term = __int_as_float(0x7fffffff);  // a term outside FP32's squares: warp 0 evaluates it
+            if (st == ST_OK) Nll::ordinary(o, pr, se2, term);
+            tm.terms[(r - c0) * 32 + lane] = term;
+        }
+        __syncthreads();
+        if (tm.warp == 0) {
+#pragma unroll 1
+            for (int r = c0; r < c1; r++) {
+                const int i = u + r * s;
+                if (i >= n) break;
+                const float term = tm.terms[(r - c0) * 32 + lane];
+                if (term == term) {
+                    acc.add(term);
+                } else {
+                    const float4 o = obs[i];
+                    int st = ST_OK;
+                    const float pr = m.eval(o.x, o.y, st);
+                    acc = Nll::obs_call(acc, o, pr, st, se2);
+                }
+            }
+        }
     }
     return acc;
 }
@@ -193,8 +264,11 @@ __device__ __forceinline__ int split_lanes(int k) {
     return s > 8 ? 8 : s;
 }
 
-template <int KIND>
-__device__ __forceinline__ double particle_cost_split(const TaskCtx& t, const float* x, int base, int k) {
+// TEAM: the whole block evaluates the round, the positions in tm->pos; warp 0
+// returns the costs.
+template <int KIND, bool TEAM = false>
+__device__ __forceinline__ double particle_cost_split(const TaskCtx& t, const float* x, int base, int k,
+                                                      const SwarmTeam* tm = nullptr) {
     const int lane = threadIdx.x & 31;
     const int s = split_lanes(k);
     const int g = lane / s, u = lane - g * s;
@@ -204,7 +278,7 @@ __device__ __forceinline__ double particle_cost_split(const TaskCtx& t, const fl
     constexpr int NX = MB ? 4 * (KIND - KIND_MB1 + 1) + 2 : n_params_of(KIND);
     float xs[NX];
 #pragma unroll
-    for (int j = 0; j < NX; j++) xs[j] = __shfl_sync(FULL_MASK, x[j], src);
+    for (int j = 0; j < NX; j++) xs[j] = TEAM ? tm->pos[j * 32 + src] : __shfl_sync(FULL_MASK, x[j], src);
     Nll acc;
     acc.reset();
     double prior = 0.0;
@@ -212,7 +286,13 @@ __device__ __forceinline__ double particle_cost_split(const TaskCtx& t, const fl
     if constexpr (MB) {
         constexpr int K = KIND - KIND_MB1 + 1;
         float se = expf(xs[4 * K + 1]);
-        if (on) acc = nll_multibazin<K>(xs, t.obs, t.n, se * se, u, s);
+        if constexpr (TEAM) {
+            MultiBazinF<K> e;
+            e.init(xs);
+            acc = nll_team(e, t.obs, on ? t.n : 0, t.n, se * se, u, s, *tm);
+        } else if (on) {
+            acc = nll_multibazin<K>(xs, t.obs, t.n, se * se, u, s);
+        }
     } else {
         constexpr int m = KIND;
         constexpr int np = n_params_of(m);
@@ -225,7 +305,7 @@ __device__ __forceinline__ double particle_cost_split(const TaskCtx& t, const fl
 #pragma unroll
             for (int i = 0; i < np; i++) p[i] = xs[i];
         }
-        if constexpr (m == VILLAR) villar_c = VillarF::constraint(p);
+        if constexpr (m == VILLAR) villar_c = VillarF::constraint_swarm(p);
         if (t.flags & TASK_PRIOR) {
             float sp = 0.0f;
 #pragma unroll
@@ -240,16 +320,25 @@ __device__ __forceinline__ double particle_cost_split(const TaskCtx& t, const fl
         }
         float se = expf(p[se_idx_of(m)]);
         float se2 = se * se;
-        if (on && !(villar_c > 0.0f)) {
-            if constexpr (m == BAZIN) { BazinF e; e.init(p); acc = nll_loop(e, t.obs, t.n, se2, u, s); }
-            else if constexpr (m == VILLAR) { VillarF e; e.init(p); acc = nll_loop(e, t.obs, t.n, se2, u, s); }
-            else if constexpr (m == TDE) { TdeF e; e.init(p); acc = nll_loop(e, t.obs, t.n, se2, u, s); }
-            else if constexpr (m == ARNETT) { ArnettF e; e.init(p); acc = nll_loop(e, t.obs, t.n, se2, u, s); }
-            else if constexpr (m == MAGNETAR) { MagnetarF e; e.init(p); acc = nll_loop(e, t.obs, t.n, se2, u, s); }
-            else if constexpr (m == SHOCK) { ShockF e; e.init(p); acc = nll_loop(e, t.obs, t.n, se2, u, s); }
-            else if constexpr (m == AFTERGLOW) { AfterglowF e; e.init(p); acc = nll_loop(e, t.obs, t.n, se2, u, s); }
-        }
+        const bool eval = on && !(villar_c > 0.0f);
+        auto terms = [&](auto e) {
+            if constexpr (TEAM) {
+                e.init(p);
+                acc = nll_team(e, t.obs, eval ? t.n : 0, t.n, se2, u, s, *tm);
+            } else if (eval) {
+                e.init(p);
+                acc = nll_loop(e, t.obs, t.n, se2, u, s);
+            }
+        };
+        if constexpr (m == BAZIN) terms(BazinF());
+        else if constexpr (m == VILLAR) terms(VillarF());
+        else if constexpr (m == TDE) terms(TdeF());
+        else if constexpr (m == ARNETT) terms(ArnettF());
+        else if constexpr (m == MAGNETAR) terms(MagnetarF());
+        else if constexpr (m == SHOCK) terms(ShockF());
+        else if constexpr (m == AFTERGLOW) terms(AfterglowF());
     }
+    if (TEAM && tm->warp != 0) return 0.0;
     double tot;
     float big;
     int nonfinite, inf;
