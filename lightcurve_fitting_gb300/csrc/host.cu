@@ -169,6 +169,7 @@ struct lcf_ctx {
     int cand_bps_rest[N_TUNE] = {1, 1, 1};  // blocks per SM, the other swarms
     int max_pso_warps_per_sm = 1;
     int lb_grid = 1;          // blocks of the persistent polish grid
+    int team_obs0 = TEAM_NEVER, team_obs = TEAM_NEVER;  // block-run swarms (is_team_task)
     int lb_n_long = 0;        // bands of LB_LONG_OBS observations or more
     int lb_n_mid = 0;         // bands polished by a whole warp (polish_warp_obs observations or more)
     int cfg = 0;             // candidate of the current fit
@@ -182,10 +183,10 @@ struct lcf_ctx {
     // after the polish and BIC selection)
     cudaStream_t stream_mb = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-    int mb_branch = 1;
     // the MetzgerKN bands' uncertainty and refinements, beside the other bands'
     cudaStream_t stream_kn = nullptr;
     cudaEvent_t ev_fork_kn = nullptr, ev_join_kn = nullptr;
+    int mb_branch = 1;
     bool mb_timed = false;   // the last enqueued sequence recorded ev[9], ev[10]
     bool mb_branched = false;  // ... and ran MultiBazin on its branch
     std::string err;
@@ -314,10 +315,10 @@ extern "C" int lcf_ctx_create(int device, lcf_ctx** out) {
     if (cudaStreamCreateWithFlags(&ctx->stream_mb, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&ctx->ev_done, cudaEventDisableTiming) != cudaSuccess) {
         cudaStreamCreateWithFlags(&ctx->stream_kn, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->ev_fork_kn, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->ev_join_kn, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&ctx->ev_done, cudaEventDisableTiming) != cudaSuccess) {
         lcf_ctx_destroy(ctx);
         return LCF_E_CUDA;
     }
@@ -342,11 +343,11 @@ extern "C" int lcf_ctx_create(int device, lcf_ctx** out) {
     ctx->pso_blocks_per_sm = ctx->cand_bps[0];
     ctx->pso_rest_per_sm = ctx->cand_bps_rest[0];
     ctx->lb_grid = lbfgs_grid(ctx->num_sms);
-    // RNG tables
     if (finalize_init_attributes() != 0) {
         lcf_ctx_destroy(ctx);
         return LCF_E_CUDA;
     }
+    // RNG tables
     std::vector<float> draws((size_t)3 * DRAWS_PER_SEED);
     // the SVI noise, then Adam's bias corrections 1 / (1 - 0.9^t) and
     // 1 / (1 - 0.999^t) for t = 1 .. SVI_STEPS (the powers by the repeated FP64
@@ -408,10 +409,10 @@ extern "C" void lcf_ctx_destroy(lcf_ctx* ctx) {
         if (ctx->ev[i]) cudaEventDestroy(ctx->ev[i]);
     if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
     if (ctx->ev_join) cudaEventDestroy(ctx->ev_join);
-    if (ctx->stream_mb) cudaStreamDestroy(ctx->stream_mb);
     if (ctx->ev_fork_kn) cudaEventDestroy(ctx->ev_fork_kn);
     if (ctx->ev_join_kn) cudaEventDestroy(ctx->ev_join_kn);
     if (ctx->stream_kn) cudaStreamDestroy(ctx->stream_kn);
+    if (ctx->stream_mb) cudaStreamDestroy(ctx->stream_mb);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
 }
@@ -459,14 +460,6 @@ static uint64_t hash_layout(const std::vector<int64_t>& boff, const std::vector<
     mix((uint64_t)o.run_multi_bazin + 11);
     mix((uint64_t)o.joint_multiband + 13);
     return h;
-}
-
-// Estimated cost of a PSO task, in observation evaluations, for the
-// longest-first order of the work queue.
-static double task_cost(int kind, int n) {
-    if (kind == METZGER) return 330.0 + 0.8 * n;
-    if (kind >= KIND_MB1) return 0.9 * n * (kind - KIND_MB1 + 1);
-    return (double)n;
 }
 
 // Shape bucket of a batch: ceil(log2) of the band count, and of the
@@ -536,6 +529,16 @@ static void record_launch(lcf_ctx* ctx) {
     ctx->exploring = false;
 }
 
+// The shortest length of which the batch has at most `most` bands or longer.
+static int team_length(const std::vector<int64_t>& boff, int n_bands, int most) {
+    for (int len = 32; len <= 512; len *= 2) {
+        int n = 0;
+        for (int b = 0; b < n_bands; b++) n += boff[b + 1] - boff[b] >= len ? 1 : 0;
+        if (n <= most) return len;
+    }
+    return TEAM_NEVER;
+}
+
 static int prepare_layout(lcf_ctx* ctx, int n_sources, int n_bands, int64_t n_obs, const lcf_fit_options& o) {
     uint64_t key = hash_layout(ctx->h_boff, ctx->h_soff, o);
     bool same = key == ctx->layout_key && ctx->n_bands == n_bands && ctx->n_obs == n_obs;
@@ -550,9 +553,17 @@ static int prepare_layout(lcf_ctx* ctx, int n_sources, int n_bands, int64_t n_ob
         const int64_t nb_obs = ctx->h_boff[b + 1] - ctx->h_boff[b];
         n_max = std::max<int64_t>(n_max, nb_obs);
         n_long += nb_obs >= LB_LONG_OBS ? 1 : 0;
+        n_mid += nb_obs >= warp_obs ? 1 : 0;
     }
     ctx->n_max = n_max;
     ctx->lb_n_long = n_long;
+    ctx->lb_n_mid = n_mid;
+    // Swarms run by whole blocks (pso.cu): a block costs more than eight warps
+    // do, so only the few longest bands, which a launch would otherwise wait
+    // for, up to a few per SM (24 swarms a band in model selection, 3 to 8 a
+    // source in the later launches)
+    ctx->team_obs0 = team_length(ctx->h_boff, n_bands, 64);
+    ctx->team_obs = team_length(ctx->h_boff, n_bands, 300);
     // capacity
     size_t nb = (size_t)std::max(n_bands, 1), no = (size_t)std::max<int64_t>(n_obs, 1);
     int rc = 0;
@@ -566,11 +577,9 @@ static int prepare_layout(lcf_ctx* ctx, int n_sources, int n_bands, int64_t n_ob
     rc |= grow(ctx, ctx->t64, no * 8);
     rc |= grow(ctx, ctx->f64, no * 8);
     rc |= grow(ctx, ctx->fe64, no * 8);
-        n_mid += nb_obs >= warp_obs ? 1 : 0;
     rc |= grow(ctx, ctx->var64, no * 8);
     rc |= grow(ctx, ctx->uf64, no * 8);
     rc |= grow(ctx, ctx->mag64, no * 8);
-    ctx->lb_n_mid = n_mid;
     rc |= grow(ctx, ctx->up, no);
     rc |= grow(ctx, ctx->ffa, no * sizeof(float4));
     rc |= grow(ctx, ctx->ffb, no * sizeof(float2));
@@ -660,62 +669,62 @@ static int prepare_layout(lcf_ctx* ctx, int n_sources, int n_bands, int64_t n_ob
                                ctx->stream));
             CK(cudaStreamSynchronize(ctx->stream));
         }
+        // Queue order: the tasks that whole blocks run first (pso.cu takes them
+        // so), then grouped by task kind so that the warps resident on an SM at
+        // any moment run the same model's code (one kind's loop stays in the
+        // instruction cache), the costliest kind (MetzgerKN) first, and longest
+        // bands first within a kind (longest-processing-time order).  Only the
+        // bands are sorted; the tasks are written in their order (720,000 tasks
+        // of 10,000 sources: the fit's host time falls from 65 to 15 ms)
+        std::vector<int32_t> order;
+        order.reserve((size_t)n_bands);
+        for (int b = 0; b < n_bands; b++)
+            if (ctx->h_boff[b + 1] > ctx->h_boff[b]) order.push_back(b);
+        auto len = [&](int b) { return (int)(ctx->h_boff[b + 1] - ctx->h_boff[b]); };
+        std::stable_sort(order.begin(), order.end(), [&](int32_t x, int32_t y) { return len(x) > len(y); });
+        std::vector<uint8_t> joint_band((size_t)std::max(n_bands, 1), 0);
+        if (ctx->n_joint > 0)
+            for (int sidx = 0; sidx < n_sources; sidx++)
+                if (jflag[sidx])
+                    for (int b = ctx->h_soff[sidx]; b < ctx->h_soff[sidx + 1]; b++) joint_band[b] = 1;
         std::vector<PsoTask>& T = ctx->h_tasks0;
         T.clear();
-        int64_t mb_base = (int64_t)n_bands * 32;
-        for (int b = 0; b < n_bands; b++) {
-            int n = (int)(ctx->h_boff[b + 1] - ctx->h_boff[b]);
-            if (n <= 0) continue;
-            int sidx = (int)(std::upper_bound(ctx->h_soff.begin(), ctx->h_soff.end(), b) - ctx->h_soff.begin()) - 1;
-            const bool joint = ctx->n_joint > 0 && jflag[sidx];
-            int models[8], nm = 0;
-            if (joint) nm = 0;  // fitted by the joint multi-band swarm
-            else if (o.forced_model >= 0) models[nm++] = o.forced_model;
-            else if (o.fit_all_models) for (int m = 0; m < 8; m++) models[nm++] = m;
-            else models[nm++] = BAZIN;
-            for (int i = 0; i < nm; i++)
-                for (int r = 0; r < 3; r++) {
-                    PsoTask t;
-                    t.band = b;
-                    t.kind = (int16_t)models[i];
-                    t.restart = (int8_t)r;
-                    t.flags = TASK_PRIOR | TASK_T0_BOUNDS | (r > 0 ? TASK_SEEDED : 0);
-                    t.out = (b * 8 + models[i]) * 3 + r;
-                    t.aux = -1;
-                    t.t0_fixed = 0.0;
-                    T.push_back(t);
-                }
-            if (o.run_multi_bazin && n >= 5)
+        T.reserve(order.size() * 26);
+        const int64_t mb_base = (int64_t)n_bands * 32;
+        auto fitted = [&](int kind) {
+            return o.forced_model >= 0 ? kind == o.forced_model : o.fit_all_models ? true : kind == BAZIN;
+        };
+        auto add = [&](int kind, int b) {
+            const int n = len(b);
+            PsoTask t;
+            t.band = b;
+            t.kind = (int16_t)kind;
+            t.aux = -1;
+            t.t0_fixed = 0.0;
+            if (kind == KIND_MB1) {
+                if (!o.run_multi_bazin || n < 5) return;
                 for (int r = 0; r < 3; r += 2) {
-                    PsoTask t;
-                    t.band = b;
-                    t.kind = (int16_t)KIND_MB1;
                     t.restart = (int8_t)r;
                     t.flags = TASK_RANK0;
                     t.out = (int)(mb_base + ((int64_t)b * 4) * 3 + r);
-                    t.aux = -1;
-                    t.t0_fixed = 0.0;
                     T.push_back(t);
                 }
-        }
-        // Queue order: grouped by task kind so that the warps resident on an
-        // SM at any moment run the same model's code (one kind's loop stays in
-        // the instruction cache), the costliest kind (MetzgerKN) first, and
-        // longest bands first within a kind (longest-processing-time order).
-        std::vector<double> key(T.size());
-        for (size_t i = 0; i < T.size(); i++)
-            key[i] = task_cost(T[i].kind, (int)(ctx->h_boff[T[i].band + 1] - ctx->h_boff[T[i].band]));
-        auto group = [](int kind) { return kind == METZGER ? 0 : 1 + kind; };
-        std::vector<size_t> ord(T.size());
-        for (size_t i = 0; i < ord.size(); i++) ord[i] = i;
-        std::stable_sort(ord.begin(), ord.end(), [&](size_t a, size_t b) {
-            int ga = group(T[a].kind), gb = group(T[b].kind);
-            if (ga != gb) return ga < gb;
-            return key[a] > key[b];
-        });
-        std::vector<PsoTask> S(T.size());
-        for (size_t i = 0; i < ord.size(); i++) S[i] = T[ord[i]];
-        T.swap(S);
+                return;
+            }
+            // a joint band is fitted by the joint multi-band swarm
+            if (joint_band[b] || !fitted(kind)) return;
+            for (int r = 0; r < 3; r++) {
+                t.restart = (int8_t)r;
+                t.flags = TASK_PRIOR | TASK_T0_BOUNDS | (r > 0 ? TASK_SEEDED : 0);
+                t.out = (b * 8 + kind) * 3 + r;
+                T.push_back(t);
+            }
+        };
+        static const int kinds[9] = {METZGER, BAZIN, VILLAR, TDE, ARNETT, MAGNETAR, SHOCK, AFTERGLOW, KIND_MB1};
+        for (int team = 1; team >= 0; team--)
+            for (int kind : kinds)
+                for (int32_t b : order)
+                    if ((is_team_task(kind, len(b), ctx->team_obs0) ? 1 : 0) == team) add(kind, b);
         ctx->n_tasks0 = (int)T.size();
         CK(cudaMemcpyAsync(ctx->tasks[0].p, T.data(), T.size() * sizeof(PsoTask), cudaMemcpyHostToDevice,
                            ctx->stream));
@@ -736,6 +745,7 @@ static int prepare_layout(lcf_ctx* ctx, int n_sources, int n_bands, int64_t n_ob
     d.src_off = (const int32_t*)ctx->soff.p;
     d.n_sources = n_sources;
     d.n_bands = n_bands;
+    d.num_sms = ctx->num_sms;
     d.n_obs = n_obs;
     d.stats = (BandStats*)ctx->stats_b.p;
     d.obs = (float4*)ctx->obs.p;
@@ -758,7 +768,6 @@ static int prepare_layout(lcf_ctx* ctx, int n_sources, int n_bands, int64_t n_ob
     d.out = (BandOut*)ctx->out.p;
     d.mb = (MbState*)ctx->mb.p;
     for (int s = 0; s < 7; s++) {
-    d.num_sms = ctx->num_sms;
         d.tasks[s] = (PsoTask*)ctx->tasks[s].p;
         d.task_cap[s] = (int)ctx->task_cap[s];
     }
@@ -770,6 +779,9 @@ static int prepare_layout(lcf_ctx* ctx, int n_sources, int n_bands, int64_t n_ob
     d.polish_order = (int32_t*)ctx->polish_order.p;
     d.lb_grid = ctx->lb_grid;
     d.lb_n_long = ctx->lb_n_long;
+    d.lb_n_mid = ctx->lb_n_mid;
+    d.team_obs0 = ctx->team_obs0;
+    d.team_obs = ctx->team_obs;
     d.n_joint = ctx->n_joint;
     d.joint_flag = ctx->n_joint > 0 ? (const uint8_t*)ctx->joint_flag.p : nullptr;
     d.joint_src = (const int32_t*)ctx->joint_src.p;
@@ -792,7 +804,6 @@ static int prepare_layout(lcf_ctx* ctx, int n_sources, int n_bands, int64_t n_ob
     d.mb_slot_base = (int64_t)n_bands * 32;
     d.smem_obs = ctx->smem_obs;
     d.wait_polls = ctx->wait_polls;
-    d.lb_n_mid = ctx->lb_n_mid;
     return 0;
 }
 
@@ -808,17 +819,6 @@ static void stage_event(lcf_ctx* ctx, cudaEvent_t e, cudaStream_t q) {
     else cudaEventRecord(e, q);
 }
 
-static void enqueue_pipeline(lcf_ctx* ctx) {
-    const DeviceBatch& d = ctx->db;
-    const lcf_fit_options& o = ctx->opts;
-    cudaStream_t s = ctx->stream;
-    int grid0 = ctx->num_sms * ctx->pso_blocks_per_sm;
-    int grid = ctx->num_sms * ctx->pso_rest_per_sm;
-    int block = ctx->pso_block;
-    int64_t L = 0;
-    stage_event(ctx, ctx->ev[0], s);
-    cudaMemsetAsync(ctx->res.p, 0xff, (size_t)std::max(ctx->n_bands, 1) * 44 * sizeof(PsoResult), s);
-    cudaMemsetAsync(ctx->ctr.p, 0, sizeof(Counters), s);
 // The MetzgerKN bands' uncertainty (unless it was given) and refinements on
 // their own stream: a few bands whose chains of ODE steps are far longer than
 // the other models' run beside those instead of before them.  The caller joins
@@ -837,6 +837,17 @@ static int enqueue_metzger(lcf_ctx* ctx, bool uncertainty) {
     return uncertainty ? 2 : 1;
 }
 
+static void enqueue_pipeline(lcf_ctx* ctx) {
+    const DeviceBatch& d = ctx->db;
+    const lcf_fit_options& o = ctx->opts;
+    cudaStream_t s = ctx->stream;
+    int grid0 = ctx->num_sms * ctx->pso_blocks_per_sm;
+    int grid = ctx->num_sms * ctx->pso_rest_per_sm;
+    int block = ctx->pso_block;
+    int64_t L = 0;
+    stage_event(ctx, ctx->ev[0], s);
+    cudaMemsetAsync(ctx->res.p, 0xff, (size_t)std::max(ctx->n_bands, 1) * 44 * sizeof(PsoResult), s);
+    cudaMemsetAsync(ctx->ctr.p, 0, sizeof(Counters), s);
     cudaMemsetAsync(ctx->fits.p, 0xff, (size_t)std::max(ctx->n_bands, 1) * 8 * sizeof(ModelFit), s);
     launch_prep(d, s); L++;
     stage_event(ctx, ctx->ev[1], s);
@@ -898,6 +909,7 @@ static int enqueue_metzger(lcf_ctx* ctx, bool uncertainty) {
     L++;
     stage_event(ctx, ctx->ev[5], s);
     launch_refine(d, s); L++;
+    cudaStreamWaitEvent(s, ctx->ev_join_kn, 0);
     stage_event(ctx, ctx->ev[6], s);
     if (o.run_multi_bazin && branch == 0) enqueue_mb(s);
     if (branch) cudaStreamWaitEvent(s, ctx->ev_join, 0);
@@ -909,7 +921,6 @@ static int run_pipeline(lcf_ctx* ctx) {
     cudaGetLastError();  // a failed query elsewhere in the process must not be reported as ours
     // set per fit (a graph replay does not run enqueue_pipeline)
     ctx->mb_timed = ctx->opts.run_multi_bazin != 0;
-    cudaStreamWaitEvent(s, ctx->ev_join_kn, 0);
     ctx->mb_branched = ctx->mb_timed && ctx->mb_branch != 0;
     uint64_t gkey = ctx->layout_key ^ ((uint64_t)(uintptr_t)ctx->db.times * 31) ^ ((uint64_t)ctx->n_obs << 7) ^
                     ((uint64_t)(ctx->cfg + 1) << 56) ^ ((uint64_t)(ctx->mb_branch + 1) << 52);
@@ -1254,6 +1265,7 @@ static void enqueue_finalize(lcf_ctx* ctx, bool given, size_t sel_bytes) {
     cudaEventRecord(ctx->ev[8], s);
     launch_band_order(d, s); L++;
     cudaEventRecord(ctx->ev[4], s);
+    L += enqueue_metzger(ctx, !given);
     if (!given) {
         if (ctx->opts.method == LCF_METHOD_SVI) launch_svi(d, s);
         else launch_laplace(d, s);
@@ -1261,11 +1273,11 @@ static void enqueue_finalize(lcf_ctx* ctx, bool given, size_t sel_bytes) {
     }
     cudaEventRecord(ctx->ev[5], s);
     launch_refine(d, s); L++;
+    cudaStreamWaitEvent(s, ctx->ev_join_kn, 0);
     cudaEventRecord(ctx->ev[6], s);
     cudaEventRecord(ctx->ev[7], s);
     ctx->launches = L;
 }
-    L += enqueue_metzger(ctx, !given);
 
 extern "C" int lcf_finalize_batch(lcf_ctx* ctx, const lcf_bands_csr* in, const lcf_pso_selection* sel, int method,
                                   lcf_fit_outputs* out) {
@@ -1273,7 +1285,6 @@ extern "C" int lcf_finalize_batch(lcf_ctx* ctx, const lcf_bands_csr* in, const l
     if (int rc = busy(ctx)) return rc;
     if (!in || !sel || !out) return set_err(ctx, LCF_E_INVALID, "null argument");
     const bool given = sel->svi_mu != nullptr || sel->svi_log_sigma != nullptr;
-    cudaStreamWaitEvent(s, ctx->ev_join_kn, 0);
     if (given && !(sel->svi_mu && sel->svi_log_sigma))
         return set_err(ctx, LCF_E_INVALID, "svi_mu and svi_log_sigma are given together");
     if (!given && method != LCF_METHOD_SVI && method != LCF_METHOD_LAPLACE)

@@ -155,6 +155,13 @@ enum : uint8_t {
     TASK_RANK0 = 16,      // run only if the band is its source's rank-0 band with n >= 5
 };
 
+// A swarm task that a whole block runs (pso.cu): every model but MetzgerKN,
+// whose cost is its particles' ODEs, on a band of team_obs observations or more.
+constexpr int TEAM_NEVER = 1 << 30;
+__host__ __device__ inline bool is_team_task(int kind, int n, int team_obs) {
+    return kind != METZGER && n >= team_obs;
+}
+
 // Result of one PSO run.
 struct PsoResult {
     double cost;
@@ -229,6 +236,7 @@ struct Counters {
     int32_t polish_hist[256];   // bands by length: histogram, then offsets (polish_order)
     int32_t lb_next[8];         // per model: next index of the polish queue (eight lanes a band)
     int32_t lb_next_long[8];    // per model: next index of its long bands (a warp a band)
+    int32_t lb_next_mid[8];     // per model: next index of its middle bands (a warp a band, eight-lane order)
     int32_t error;              // first error code raised on the device
     int32_t joint_head;         // next (source, restart) task of the joint multi-band swarm
 };
@@ -236,12 +244,12 @@ struct Counters {
 struct DeviceBatch {
     // raw inputs (FP64, caller layout)
     const double* times;
-    int32_t lb_next_mid[8];     // per model: next index of its middle bands (a warp a band, eight-lane order)
     const double* flux;
     const double* err;
     const int64_t* band_off;
     const int32_t* src_off;
     int n_sources, n_bands;
+    int num_sms;
     int64_t n_obs;
     // prepared
     BandStats* stats;
@@ -249,7 +257,6 @@ struct DeviceBatch {
     double* t64;            // [n_obs] sorted FP64 copies for the FP64 stages
     double* f64;            // flux / peak
     double* fe64;           // err / peak
-    int num_sms;
     double* var64;          // obs_var
     double* uf64;           // upper flux
     double* mag64;          // observed magnitude
@@ -280,6 +287,7 @@ struct DeviceBatch {
     int32_t* polish_order;  // [n_bands] bands longest first: the polish's queue order
     int lb_grid;            // blocks of the persistent polish grid
     int lb_n_long;          // bands of LB_LONG_OBS observations or more (the first of polish_order)
+    int lb_n_mid;           // bands polished by a whole warp (the first of polish_order; >= lb_n_long)
     Counters* ctr;
     float* scratch;         // MetzgerKN per-warp scratch: [warps][n_max][32]
     int64_t scratch_per_warp;
@@ -287,9 +295,9 @@ struct DeviceBatch {
     float* scratch_svi;     // MetzgerKN SVI scratch, 20 values per observation
     double* t0_state;       // per band: t0_min, t0_max, best t0 of the profile search
     int64_t t0_slot_base;   // first PsoResult slot of the t0 search region
-    int lb_n_mid;           // bands polished by a whole warp (the first of polish_order; >= lb_n_long)
     int64_t mb_slot_base;   // first PsoResult slot of the MultiBazin region
     int smem_obs;           // observations staged per warp in the PSO kernel
+    int team_obs0, team_obs;  // is_team_task's length: the model-selection launch, the other swarm launches
     int wait_polls;         // bound of the staging copy's barrier wait, in polls (lcf_set_wait_bound)
     // joint multi-band fit
     const uint8_t* joint_flag;   // per source: 1 if fitted jointly
@@ -334,6 +342,9 @@ void launch_mb_build(const DeviceBatch& d, int slot, int k, cudaStream_t s);
 void launch_lbfgs(const DeviceBatch& d, int model_mask, cudaStream_t s);
 // Bands of at least this many observations are polished by a whole warp.
 constexpr int LB_LONG_OBS = 256;
+// Bands of at least this many observations (a multiple of 8, at most
+// LB_LONG_OBS) are polished by a whole warp.
+int polish_warp_obs(int n_bands, int lb_grid);
 // the polish queue's band order (three launches); before the first launch_lbfgs
 void launch_polish_order(const DeviceBatch& d, cudaStream_t s);
 // blocks of the persistent polish grid on `num_sms` SMs
@@ -342,9 +353,6 @@ void launch_select(const DeviceBatch& d, int fit_all, int forced, cudaStream_t s
 void launch_svi(const DeviceBatch& d, cudaStream_t s);
 // one SVI step's ELBO estimate and gradient at given variational parameters
 // (lcf_svi_elbo_grad); scratch = 5 n floats per point
-// Bands of at least this many observations (a multiple of 8, at most
-// LB_LONG_OBS) are polished by a whole warp.
-int polish_warp_obs(int n_bands, int lb_grid);
 void launch_svi_grad(int model, const float4* obs, int n, float t_last, const double* init, const double* vpar,
                      int n_points, const double* eps, int n_samples, double* elbo, double* grad, int* flags,
                      float* scratch, cudaStream_t s);
@@ -360,6 +368,12 @@ void launch_laplace(const DeviceBatch& d, cudaStream_t s);
 // bands grouped by selected model into d.band_order, their counts into ctr->band_hist
 void launch_band_order(const DeviceBatch& d, cudaStream_t s);
 void launch_refine(const DeviceBatch& d, cudaStream_t s);
+// the MetzgerKN bands of SVI, Laplace and the refinements, which the kernels
+// above leave out (after launch_band_order)
+void launch_svi_metzger(const DeviceBatch& d, cudaStream_t s);
+void launch_laplace_metzger(const DeviceBatch& d, cudaStream_t s);
+void launch_refine_metzger(const DeviceBatch& d, cudaStream_t s);
+int finalize_init_attributes();
 double probe_fp32_tflops(int num_sms);
 // polish.cu: FP64 peaks: out[m] = observation-term evaluations per second of
 // the polish's FP64 cost+gradient term for model m (0..6) at full occupancy,
@@ -368,12 +382,6 @@ int probe_fp64_peaks(int num_sms, double* out9);
 int probe_ff(int num_sms, double* out80);
 double probe_mufu_gops(int num_sms);
 void launch_band_cost(int model, const float4* obs, int n, float t_last, const double* params, int n_eval,
-// the MetzgerKN bands of SVI, Laplace and the refinements, which the kernels
-// above leave out (after launch_band_order)
-void launch_svi_metzger(const DeviceBatch& d, cudaStream_t s);
-void launch_laplace_metzger(const DeviceBatch& d, cudaStream_t s);
-void launch_refine_metzger(const DeviceBatch& d, cudaStream_t s);
-int finalize_init_attributes();
                       int with_prior, double* costs, float* scratch, cudaStream_t s);
 
 // Host-side generation of the RNG tables (host.cpp)

@@ -270,6 +270,27 @@ struct WarpSmemOf<7> {
     using type = WarpSmem;
 };
 
+// A block's swarm (swarm_cost.cuh): warp 0 hands the round over (the positions
+// and the first particle, or -1 at the swarm's end), the other warps wait for
+// it and evaluate their share.
+template <int D>
+__device__ __forceinline__ void team_round(const float* x, int start, const SwarmTeam& tm, int* cmd) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int k = 0; k < D; k++) tm.pos[32 * k + lane] = x[k];
+    if (lane == 0) *cmd = start;
+    __syncthreads();
+}
+template <int KIND>
+__device__ __noinline__ void team_worker(const TaskCtx& t, const SwarmTeam& tm, const int* cmd) {
+    while (true) {
+        __syncthreads();
+        const int start = *cmd;
+        if (start < 0) return;
+        particle_cost_split<KIND, true>(t, nullptr, start, NP - start, &tm);
+    }
+}
+
 // One swarm run (pso_minimize / pso_minimize_seeded, src/parametric.rs:1646-1757,
 // 1160-1266) of a task of kind KIND: warp = swarm, lane = particle.
 template <int MAXD, int KIND>
@@ -553,9 +574,10 @@ __device__ __forceinline__ void exact_cost_setup(LaneLb<KIND>& lc, const DeviceB
     lc.with_prior = (flags & TASK_PRIOR) != 0;
 }
 
-template <int KIND>
+template <int KIND, bool TEAM>
 __device__ __forceinline__ void run_swarm_exact(const DeviceBatch& d, const PsoTask& task, const BandStats& bs,
-                                                TaskCtx& t, WarpSmem* ws, int slot) {
+                                                TaskCtx& t, WarpSmem* ws, int slot, const SwarmTeam* tm = nullptr,
+                                                int* cmd = nullptr) {
     constexpr int m = KIND, np = n_params_of(m), t0i = t0_idx_of(m), MAXD = 7;
     const int lane = threadIdx.x & 31;
     const int p = lane;
@@ -668,7 +690,8 @@ __device__ __forceinline__ void run_swarm_exact(const DeviceBatch& d, const PsoT
     // one evaluation round over lanes start .. NP - 1 (lane-split FP32)
     auto eval_round = [&](int start) -> double {
         const int kk = NP - start;
-        const double cs = particle_cost_split<KIND>(t, xh, start, kk);
+        if constexpr (TEAM) team_round<MAXD>(xh, start, *tm, cmd);
+        const double cs = particle_cost_split<KIND, TEAM>(t, xh, start, kk, tm);
         const double co = __shfl_sync(FULL, cs, ((p - start) * split_lanes(kk)) & 31);
         return (live && p >= start) ? co : INFINITY;
     };
@@ -877,10 +900,11 @@ __device__ __noinline__ double mb_cost_fp64(const DeviceBatch& d, const BandStat
 // One extra move per particle and iteration; 18 dimensions need 7.5 KB of
 // shared memory a warp instead of 12.1 KB.
 // ---------------------------------------------------------------------------
-template <int MAXD, int KIND>
+template <int MAXD, int KIND, bool TEAM>
 __device__ __forceinline__ void run_swarm_exact_mb(const DeviceBatch& d, const PsoTask& task, const BandStats& bs,
                                                    TaskCtx& t, ff* s_lo, ff* s_hi, ff* s_vm, ff* s_g, float* st,
-                                                   double* s_pos, int slot) {
+                                                   double* s_pos, int slot, const SwarmTeam* tm = nullptr,
+                                                   int* cmd = nullptr) {
     constexpr int K = KIND - KIND_MB1 + 1, D = 4 * K + 2;
     static_assert(D <= MAXD, "MultiBazin swarm wider than the instantiation");
     const int lane = threadIdx.x & 31;
@@ -955,7 +979,8 @@ __device__ __forceinline__ void run_swarm_exact_mb(const DeviceBatch& d, const P
     // one evaluation round over lanes start .. NP - 1 at the trial positions
     auto eval_round = [&](int start) -> double {
         const int kk = NP - start;
-        const double cs = particle_cost_split<KIND>(t, xt, start, kk);
+        if constexpr (TEAM) team_round<D>(xt, start, *tm, cmd);
+        const double cs = particle_cost_split<KIND, TEAM>(t, xt, start, kk, tm);
         const double co = __shfl_sync(FULL, cs, ((p - start) * split_lanes(kk)) & 31);
         return (live && p >= start) ? co : INFINITY;
     };
@@ -1090,6 +1115,24 @@ __device__ __forceinline__ void run_swarm_exact_mb(const DeviceBatch& d, const P
     __syncwarp();
 }
 
+// A task run by the whole block.  Out of line: the one-warp swarms keep their
+// registers.
+template <int MAXD, int KIND>
+__device__ __noinline__ void run_team(const DeviceBatch& d, const PsoTask& task, const BandStats& bs, TaskCtx& t,
+                                      typename WarpSmemOf<MAXD>::type* ws, int slot, const SwarmTeam& tm, int* cmd) {
+    if (tm.warp != 0) {
+        team_worker<KIND>(t, tm, cmd);
+        return;
+    }
+    if constexpr (KIND >= KIND_MB1)
+        run_swarm_exact_mb<MAXD, KIND, true>(d, task, bs, t, ws->lo, ws->hi, ws->vmax, ws->g, &ws->lo_state[0][0][0],
+                                             ws->s_pos, slot, &tm, cmd);
+    else
+        run_swarm_exact<KIND, true>(d, task, bs, t, ws, slot, &tm, cmd);
+    if ((threadIdx.x & 31) == 0) *cmd = -1;
+    __syncthreads();
+}
+
 // MINB: blocks of 256 threads per SM the register budget is sized for.  Two
 // (128 registers a thread, 16 warps) is the default: measured on GB300 it runs
 // the swarms ~1.7x faster than one block without spills.  The 7-dimension
@@ -1099,7 +1142,7 @@ __device__ __forceinline__ void run_swarm_exact_mb(const DeviceBatch& d, const P
 // slower, so the launch autotuner offers it for model selection only.
 template <int MAXD, int MINB>
 __global__ void __launch_bounds__(256, MINB)
-    pso_kernel(DeviceBatch d, int slot, const PsoTask* tasks, int n_host, int smem_obs) {
+    pso_kernel(DeviceBatch d, int slot, const PsoTask* tasks, int n_host, int smem_obs, int team_obs) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -1113,16 +1156,7 @@ __global__ void __launch_bounds__(256, MINB)
     const int n_tasks = n_host >= 0 ? n_host : d.ctr->task_count[slot];
     const int gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
 
-    while (true) {
-        int ti = 0;
-        if (lane == 0) ti = atomicAdd(&d.ctr->task_head[slot], 1);
-        ti = __shfl_sync(FULL, ti, 0);
-        if (ti >= n_tasks) break;
-        const PsoTask task = tasks[ti];
-        const BandStats bs = d.stats[task.band];
-        // tasks of bands the reference does not fit (or MultiBazin tasks of
-        // bands that are not their source's rank-0 band with n >= 5) are no-ops
-        if (!bs.valid || ((task.flags & TASK_RANK0) && (bs.rank != 0 || bs.n < 5))) continue;
+    auto context = [&](const PsoTask& task, const BandStats& bs) {
         TaskCtx t;
         t.kind = task.kind;
         t.flags = task.flags;
@@ -1130,6 +1164,76 @@ __global__ void __launch_bounds__(256, MINB)
         t.inv_n = 1.0 / (double)max(bs.n, 1);
         t.t_last = (float)bs.t_last;
         t.t0_fixed = (float)task.t0_fixed;
+        return t;
+    };
+    // tasks of bands the reference does not fit (or MultiBazin tasks of
+    // bands that are not their source's rank-0 band with n >= 5) are no-ops
+    auto skip = [&](const PsoTask& task, const BandStats& bs) {
+        return !bs.valid || ((task.flags & TASK_RANK0) && (bs.rank != 0 || bs.n < 5));
+    };
+
+    // The queue's first tasks, those of bands of team_obs observations or more
+    // (is_team_task), are run one at a time by the whole block; then each warp
+    // takes tasks of its own.
+    int next = -1;  // warp 0: the first one-warp task, taken below
+    {
+        __shared__ int s_ti, s_cmd;
+        while (team_obs < TEAM_NEVER) {
+            if (threadIdx.x == 0) s_ti = atomicAdd(&d.ctr->task_head[slot], 1);
+            __syncthreads();
+            const int ti = s_ti;
+            if (ti >= n_tasks) return;
+            const PsoTask task = tasks[ti];
+            const BandStats bs = d.stats[task.band];
+            if (!is_team_task(task.kind, bs.n, team_obs)) {
+                if (warp == 0) next = ti;
+                break;
+            }
+            if (!skip(task, bs)) {
+                TaskCtx t = context(task, bs);
+                // the block's staging memory: positions, terms, the band
+                SwarmTeam tm;
+                tm.pos = reinterpret_cast<float*>(smem_raw);
+                tm.terms = tm.pos + 32 * MAXD;
+                tm.warp = warp;
+                tm.n_warps = nwarps;
+                float4* band = reinterpret_cast<float4*>(tm.terms + 32 * TEAM_ROWS);
+                const int cap = nwarps * smem_obs - (32 * MAXD + 32 * TEAM_ROWS) / 4;
+                t.obs = d.obs + bs.off;
+                if (bs.n <= cap) {
+                    for (int i = threadIdx.x; i < bs.n; i += blockDim.x) band[i] = t.obs[i];
+                    t.obs = band;
+                }
+                __syncthreads();
+                if constexpr (MAXD != 7) {
+                    run_team<MAXD, KIND_MB1 + (MAXD - 2) / 4 - 1>(d, task, bs, t, ws, slot, tm, &s_cmd);
+                } else switch (task.kind) {
+                    case BAZIN: run_team<7, BAZIN>(d, task, bs, t, ws, slot, tm, &s_cmd); break;
+                    case VILLAR: run_team<7, VILLAR>(d, task, bs, t, ws, slot, tm, &s_cmd); break;
+                    case TDE: run_team<7, TDE>(d, task, bs, t, ws, slot, tm, &s_cmd); break;
+                    case ARNETT: run_team<7, ARNETT>(d, task, bs, t, ws, slot, tm, &s_cmd); break;
+                    case MAGNETAR: run_team<7, MAGNETAR>(d, task, bs, t, ws, slot, tm, &s_cmd); break;
+                    case SHOCK: run_team<7, SHOCK>(d, task, bs, t, ws, slot, tm, &s_cmd); break;
+                    case AFTERGLOW: run_team<7, AFTERGLOW>(d, task, bs, t, ws, slot, tm, &s_cmd); break;
+                    default: run_team<7, KIND_MB1>(d, task, bs, t, ws, slot, tm, &s_cmd); break;
+                }
+            }
+            __syncthreads();  // the task, the band and the command are free again
+        }
+    }
+
+    while (true) {
+        int ti = next;
+        next = -1;
+        if (ti < 0) {
+            if (lane == 0) ti = atomicAdd(&d.ctr->task_head[slot], 1);
+            ti = __shfl_sync(FULL, ti, 0);
+        }
+        if (ti >= n_tasks) break;
+        const PsoTask task = tasks[ti];
+        const BandStats bs = d.stats[task.band];
+        if (skip(task, bs)) continue;
+        TaskCtx t = context(task, bs);
         // stage the band
         const float4* gobs = d.obs + bs.off;
         if (bs.n <= smem_obs && bs.n > 0) {
@@ -1158,19 +1262,19 @@ __global__ void __launch_bounds__(256, MINB)
         if constexpr (MAXD != 7) {
             constexpr int KMB = KIND_MB1 + (MAXD - 2) / 4 - 1;  // D = 4K + 2
             if (task.kind == KMB)
-                run_swarm_exact_mb<MAXD, KMB>(d, task, bs, t, ws->lo, ws->hi, ws->vmax, ws->g, &ws->lo_state[0][0][0],
+                run_swarm_exact_mb<MAXD, KMB, false>(d, task, bs, t, ws->lo, ws->hi, ws->vmax, ws->g, &ws->lo_state[0][0][0],
                                               ws->s_pos, slot);
         } else switch (task.kind) {
-            case BAZIN: run_swarm_exact<BAZIN>(d, task, bs, t, ws, slot); break;
-            case VILLAR: run_swarm_exact<VILLAR>(d, task, bs, t, ws, slot); break;
-            case TDE: run_swarm_exact<TDE>(d, task, bs, t, ws, slot); break;
-            case ARNETT: run_swarm_exact<ARNETT>(d, task, bs, t, ws, slot); break;
-            case MAGNETAR: run_swarm_exact<MAGNETAR>(d, task, bs, t, ws, slot); break;
-            case SHOCK: run_swarm_exact<SHOCK>(d, task, bs, t, ws, slot); break;
-            case AFTERGLOW: run_swarm_exact<AFTERGLOW>(d, task, bs, t, ws, slot); break;
+            case BAZIN: run_swarm_exact<BAZIN, false>(d, task, bs, t, ws, slot); break;
+            case VILLAR: run_swarm_exact<VILLAR, false>(d, task, bs, t, ws, slot); break;
+            case TDE: run_swarm_exact<TDE, false>(d, task, bs, t, ws, slot); break;
+            case ARNETT: run_swarm_exact<ARNETT, false>(d, task, bs, t, ws, slot); break;
+            case MAGNETAR: run_swarm_exact<MAGNETAR, false>(d, task, bs, t, ws, slot); break;
+            case SHOCK: run_swarm_exact<SHOCK, false>(d, task, bs, t, ws, slot); break;
+            case AFTERGLOW: run_swarm_exact<AFTERGLOW, false>(d, task, bs, t, ws, slot); break;
             case METZGER: run_swarm<MAXD, METZGER>(d, task, bs, t, slot, gwarp); break;
             case KIND_MB1:
-                run_swarm_exact_mb<MAXD, KIND_MB1>(d, task, bs, t, ws->lo, ws->hi, ws->vmax, ws->g,
+                run_swarm_exact_mb<MAXD, KIND_MB1, false>(d, task, bs, t, ws->lo, ws->hi, ws->vmax, ws->g,
                                                    &ws->lo_state[0][0][0], ws->s_pos, slot);
                 break;
             default: break;
@@ -1282,14 +1386,18 @@ int pso_blocks_per_sm(int block, size_t smem, int minb) {
 
 void launch_pso(const DeviceBatch& d, int slot, const PsoTask* tasks, int n_host, int max_dim, int grid, int block,
                 cudaStream_t s, int minb) {
+    int team = slot == 0 ? d.team_obs0 : d.team_obs;
+    static_assert(TEAM_ROWS * 32 % 4 == 0, "the staged band follows the terms");
     if (n_host == 0) return;
     const int smem_obs = pso_stage_obs(block, d.smem_obs, max_dim);
     const size_t smem = pso_smem_bytes(block, d.smem_obs, max_dim);
-    if (max_dim <= 7 && minb == 3) pso_kernel<7, 3><<<grid, block, smem, s>>>(d, slot, tasks, n_host, smem_obs);
-    else if (max_dim <= 7) pso_kernel<7, 2><<<grid, block, smem, s>>>(d, slot, tasks, n_host, smem_obs);
-    else if (max_dim <= 10) pso_kernel<10, 2><<<grid, block, smem, s>>>(d, slot, tasks, n_host, smem_obs);
-    else if (max_dim <= 14) pso_kernel<14, 2><<<grid, block, smem, s>>>(d, slot, tasks, n_host, smem_obs);
-    else pso_kernel<18, 2><<<grid, block, smem, s>>>(d, slot, tasks, n_host, smem_obs);
+    // a block-run swarm's positions and terms have to fit the staging memory
+    if ((block / 32) * smem_obs * 4 < 32 * (std::max(max_dim, 7) + TEAM_ROWS)) team = TEAM_NEVER;
+    if (max_dim <= 7 && minb == 3) pso_kernel<7, 3><<<grid, block, smem, s>>>(d, slot, tasks, n_host, smem_obs, team);
+    else if (max_dim <= 7) pso_kernel<7, 2><<<grid, block, smem, s>>>(d, slot, tasks, n_host, smem_obs, team);
+    else if (max_dim <= 10) pso_kernel<10, 2><<<grid, block, smem, s>>>(d, slot, tasks, n_host, smem_obs, team);
+    else if (max_dim <= 14) pso_kernel<14, 2><<<grid, block, smem, s>>>(d, slot, tasks, n_host, smem_obs, team);
+    else pso_kernel<18, 2><<<grid, block, smem, s>>>(d, slot, tasks, n_host, smem_obs, team);
 }
 
 // ---------------------------------------------------------------------------
@@ -1298,11 +1406,14 @@ void launch_pso(const DeviceBatch& d, int slot, const PsoTask* tasks, int n_host
 // the host-built model-selection queue, so that the warps resident on an SM
 // run one kind's code and the longest swarms start first.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ int task_sort_key(const PsoTask& t, int n) {
-    int grp = t.kind == METZGER ? 0 : 1 + t.kind;                      // 0..12
+// The block-run tasks (is_team_task) first, longest first and grouped by kind
+// within a length bucket; then the one-warp tasks by kind.
+__device__ __forceinline__ int task_sort_key(const PsoTask& t, int n, int team_obs) {
     int lb = (int)(2.0f * log2f((float)max(n, 1))) - 3;                // 16 length buckets
     lb = min(15, max(0, lb));
-    return grp * 16 + (15 - lb);                                       // < 208
+    if (is_team_task(t.kind, n, team_obs)) return min(15 - lb, 5) * 8 + min((int)t.kind, 7);  // < 48
+    int grp = t.kind == METZGER ? 0 : 1 + t.kind;                      // 0..12
+    return 48 + grp * 16 + (15 - lb);                                  // < 256
 }
 
 __global__ void task_hist_kernel(DeviceBatch d, int slot) {
@@ -1310,7 +1421,7 @@ __global__ void task_hist_kernel(DeviceBatch d, int slot) {
     int* hist = d.ctr->sort_hist[slot];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_tasks; i += gridDim.x * blockDim.x) {
         const PsoTask t = d.tasks[slot][i];
-        atomicAdd(&hist[task_sort_key(t, d.stats[t.band].n)], 1);
+        atomicAdd(&hist[task_sort_key(t, d.stats[t.band].n, d.team_obs)], 1);
     }
 }
 
@@ -1334,7 +1445,7 @@ __global__ void task_scatter_kernel(DeviceBatch d, int slot, PsoTask* out) {
     int* pos = d.ctr->sort_hist[slot];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_tasks; i += gridDim.x * blockDim.x) {
         const PsoTask t = d.tasks[slot][i];
-        int p = atomicAdd(&pos[task_sort_key(t, d.stats[t.band].n)], 1);
+        int p = atomicAdd(&pos[task_sort_key(t, d.stats[t.band].n, d.team_obs)], 1);
         out[p] = t;
     }
 }
