@@ -409,6 +409,7 @@ __global__ void __launch_bounds__(MZ_BLOCK) refine_metzger_kernel(DeviceBatch d)
     static_assert(NG <= MZ_SLOTS && NE < 62 && 1 + 15 <= 24, "MetzgerKN scan tables");
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n_metzger = d.ctr->band_hist[0];  // band_order's first (band_order_kernel)
+    if (tid == 0) T.lum = reinterpret_cast<double(*)[MZ_LANES]>(d.mz_lum + blockIdx.x * MZ_LUM);
     for (int ib = blockIdx.x; ib < n_metzger; ib += gridDim.x) {
         const int band = d.band_order[ib];
         const BandStats bs = d.stats[band];
@@ -791,6 +792,7 @@ __global__ void __launch_bounds__(MZ_BLOCK) laplace_metzger_kernel(DeviceBatch d
     static_assert(npts <= MZ_LANES && n_params_of(m) == np && se_idx_of(m) == ns, "MetzgerKN stencil");
     const int tid = threadIdx.x;
     const int n_metzger = d.ctr->band_hist[0];
+    if (tid == 0) T.lum = reinterpret_cast<double(*)[MZ_LANES]>(d.mz_lum + blockIdx.x * MZ_LUM);
     for (int ib = blockIdx.x; ib < n_metzger; ib += gridDim.x) {
         const int band = d.band_order[ib];
         const BandStats bs = d.stats[band];
@@ -1004,18 +1006,24 @@ void launch_refine(const DeviceBatch& d, cudaStream_t s) {
     int64_t threads = (int64_t)d.n_bands * 32;
     refine_kernel<<<(int)((threads + LCF_REFINE_BLOCK - 1) / LCF_REFINE_BLOCK), LCF_REFINE_BLOCK, 0, s>>>(d);
 }
-// The MetzgerKN bands of the refinements: one block per SM (the tables fill
-// its shared memory), the grid draining band_order's MetzgerKN bands.
+// The MetzgerKN bands of the refinements: one block per SM (the tables take
+// half of its shared memory), the grid draining band_order's MetzgerKN bands.
 void launch_refine_metzger(const DeviceBatch& d, cudaStream_t s) {
     if (d.n_bands == 0) return;
     refine_metzger_kernel<<<std::min(d.n_bands, d.num_sms), MZ_BLOCK, sizeof(MzTables), s>>>(d);
 }
 int finalize_init_attributes() {
     const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    const cudaFuncAttribute split = cudaFuncAttributePreferredSharedMemoryCarveout;  // as the SVI kernels (polish.cu)
     cudaError_t e = cudaFuncSetAttribute(refine_metzger_kernel, a, (int)sizeof(MzTables));
     if (e == cudaSuccess) e = cudaFuncSetAttribute(laplace_metzger_kernel, a, (int)sizeof(MzTables));
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(refine_metzger_kernel, split, cudaSharedmemCarveoutMaxShared);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(laplace_metzger_kernel, split, cudaSharedmemCarveoutMaxShared);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(refine_kernel, split, cudaSharedmemCarveoutMaxShared);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(laplace_kernel, split, cudaSharedmemCarveoutMaxShared);
     return (int)e;
 }
+int64_t mz_lum_doubles(int num_sms) { return (int64_t)num_sms * MZ_LUM; }
 
 // ---------------------------------------------------------------------------
 // Profile t0 search (SVI mode, rank-0 band): task builders and pickers.

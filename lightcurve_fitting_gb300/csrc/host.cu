@@ -183,9 +183,9 @@ struct lcf_ctx {
     // after the polish and BIC selection)
     cudaStream_t stream_mb = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-    // the MetzgerKN bands' uncertainty and refinements, beside the other bands'
-    cudaStream_t stream_kn = nullptr;
-    cudaEvent_t ev_fork_kn = nullptr, ev_join_kn = nullptr;
+    // the uncertainty and refinements of the models other than MetzgerKN, beside its bands'
+    cudaStream_t stream_side = nullptr;
+    cudaEvent_t ev_fork_side = nullptr, ev_join_side = nullptr;
     int mb_branch = 1;
     bool mb_timed = false;   // the last enqueued sequence recorded ev[9], ev[10]
     bool mb_branched = false;  // ... and ran MultiBazin on its branch
@@ -199,7 +199,7 @@ struct lcf_ctx {
     double* d_eps = nullptr;
     // device buffers (capacity-sized)
     DevArr times, flux, ferr, boff, soff, stats_b, obs, t64, f64, fe64, var64, uf64, mag64, up, ffa, ffb, res, fits, out, mb,
-        ctr, scratch, scratch64, scratch_svi, t0state, tasks[7], task_sorted, task_sorted_mb, band_order, polish_order, joint_flag, joint_src,
+        ctr, scratch, scratch64, scratch_svi, mz_lum, t0state, tasks[7], task_sorted, task_sorted_mb, band_order, polish_order, joint_flag, joint_src,
         joint_res, joint_draws15, joint_draws64, joint_state;
     int64_t joint_per_seed = 0;   // draws per seed held in joint_draws15
     int64_t joint_init_per_seed = 0;
@@ -315,9 +315,9 @@ extern "C" int lcf_ctx_create(int device, lcf_ctx** out) {
     if (cudaStreamCreateWithFlags(&ctx->stream_mb, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming) != cudaSuccess ||
-        cudaStreamCreateWithFlags(&ctx->stream_kn, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreateWithFlags(&ctx->ev_fork_kn, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&ctx->ev_join_kn, cudaEventDisableTiming) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&ctx->stream_side, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&ctx->ev_fork_side, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&ctx->ev_join_side, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->ev_done, cudaEventDisableTiming) != cudaSuccess) {
         lcf_ctx_destroy(ctx);
         return LCF_E_CUDA;
@@ -343,7 +343,7 @@ extern "C" int lcf_ctx_create(int device, lcf_ctx** out) {
     ctx->pso_blocks_per_sm = ctx->cand_bps[0];
     ctx->pso_rest_per_sm = ctx->cand_bps_rest[0];
     ctx->lb_grid = lbfgs_grid(ctx->num_sms);
-    if (finalize_init_attributes() != 0) {
+    if (finalize_init_attributes() != 0 || polish_init_attributes() != 0) {
         lcf_ctx_destroy(ctx);
         return LCF_E_CUDA;
     }
@@ -388,7 +388,7 @@ extern "C" void lcf_ctx_destroy(lcf_ctx* ctx) {
     if (ctx->graph) cudaGraphExecDestroy(ctx->graph);
     DevArr* all[] = {&ctx->times, &ctx->flux, &ctx->ferr, &ctx->boff, &ctx->soff, &ctx->stats_b, &ctx->obs,
                      &ctx->t64, &ctx->f64, &ctx->fe64, &ctx->var64, &ctx->uf64, &ctx->mag64, &ctx->up, &ctx->ffa, &ctx->ffb, &ctx->res,
-                     &ctx->fits, &ctx->out, &ctx->mb, &ctx->ctr, &ctx->scratch, &ctx->scratch64, &ctx->scratch_svi,
+                     &ctx->fits, &ctx->out, &ctx->mb, &ctx->ctr, &ctx->scratch, &ctx->scratch64, &ctx->scratch_svi, &ctx->mz_lum,
                      &ctx->t0state, &ctx->task_sorted, &ctx->task_sorted_mb, &ctx->band_order, &ctx->polish_order, &ctx->joint_flag,
                      &ctx->joint_src, &ctx->joint_res,
                      &ctx->joint_draws15, &ctx->joint_draws64, &ctx->joint_state,
@@ -409,9 +409,9 @@ extern "C" void lcf_ctx_destroy(lcf_ctx* ctx) {
         if (ctx->ev[i]) cudaEventDestroy(ctx->ev[i]);
     if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
     if (ctx->ev_join) cudaEventDestroy(ctx->ev_join);
-    if (ctx->ev_fork_kn) cudaEventDestroy(ctx->ev_fork_kn);
-    if (ctx->ev_join_kn) cudaEventDestroy(ctx->ev_join_kn);
-    if (ctx->stream_kn) cudaStreamDestroy(ctx->stream_kn);
+    if (ctx->ev_fork_side) cudaEventDestroy(ctx->ev_fork_side);
+    if (ctx->ev_join_side) cudaEventDestroy(ctx->ev_join_side);
+    if (ctx->stream_side) cudaStreamDestroy(ctx->stream_side);
     if (ctx->stream_mb) cudaStreamDestroy(ctx->stream_mb);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
@@ -590,6 +590,7 @@ static int prepare_layout(lcf_ctx* ctx, int n_sources, int n_bands, int64_t n_ob
     rc |= grow(ctx, ctx->ctr, sizeof(Counters));
     rc |= grow(ctx, ctx->scratch64, no * 5 * 8);
     rc |= grow(ctx, ctx->scratch_svi, no * 20 * sizeof(float));
+    rc |= grow(ctx, ctx->mz_lum, (size_t)mz_lum_doubles(ctx->num_sms) * sizeof(double));
     rc |= grow(ctx, ctx->t0state, nb * 3 * 8);
     // MetzgerKN scratch of every resident swarm warp under any candidate
     size_t warps = (size_t)ctx->num_sms * ctx->max_pso_warps_per_sm;
@@ -799,6 +800,7 @@ static int prepare_layout(lcf_ctx* ctx, int n_sources, int n_bands, int64_t n_ob
     d.scratch_per_warp = 32 * n_max;
     d.scratch64 = (double*)ctx->scratch64.p;
     d.scratch_svi = (float*)ctx->scratch_svi.p;
+    d.mz_lum = (double*)ctx->mz_lum.p;
     d.t0_state = (double*)ctx->t0state.p;
     d.t0_slot_base = (int64_t)n_bands * 24;
     d.mb_slot_base = (int64_t)n_bands * 32;
@@ -819,22 +821,32 @@ static void stage_event(lcf_ctx* ctx, cudaEvent_t e, cudaStream_t q) {
     else cudaEventRecord(e, q);
 }
 
-// The MetzgerKN bands' uncertainty (unless it was given) and refinements on
-// their own stream: a few bands whose chains of ODE steps are far longer than
-// the other models' run beside those instead of before them.  The caller joins
-// ev_join_kn.  Returns the launches.
-static int enqueue_metzger(lcf_ctx* ctx, bool uncertainty) {
+// The uncertainty (unless it was given) and the refinements.  The MetzgerKN
+// bands, a few whose chains of ODE steps are far longer than the other models',
+// run beside those: they on the context's stream, where they are placed first,
+// the others on a second one.  Records the stage events ev[5] (the other
+// models' uncertainty) and ev[6]; returns the launches.
+static int enqueue_uncertainty(lcf_ctx* ctx, bool uncertainty) {
     const DeviceBatch& d = ctx->db;
-    cudaStream_t q = ctx->stream_kn;
-    cudaEventRecord(ctx->ev_fork_kn, ctx->stream);
-    cudaStreamWaitEvent(q, ctx->ev_fork_kn, 0);
+    cudaStream_t s = ctx->stream, q = ctx->stream_side;
+    const bool svi = ctx->opts.method == LCF_METHOD_SVI;
+    cudaEventRecord(ctx->ev_fork_side, s);
+    cudaStreamWaitEvent(q, ctx->ev_fork_side, 0);
     if (uncertainty) {
-        if (ctx->opts.method == LCF_METHOD_SVI) launch_svi_metzger(d, q);
-        else launch_laplace_metzger(d, q);
+        if (svi) launch_svi_metzger(d, s);
+        else launch_laplace_metzger(d, s);
     }
-    launch_refine_metzger(d, q);
-    cudaEventRecord(ctx->ev_join_kn, q);
-    return uncertainty ? 2 : 1;
+    launch_refine_metzger(d, s);
+    if (uncertainty) {
+        if (svi) launch_svi(d, q);
+        else launch_laplace(d, q);
+    }
+    stage_event(ctx, ctx->ev[5], q);
+    launch_refine(d, q);
+    cudaEventRecord(ctx->ev_join_side, q);
+    cudaStreamWaitEvent(s, ctx->ev_join_side, 0);
+    stage_event(ctx, ctx->ev[6], s);
+    return uncertainty ? 4 : 2;
 }
 
 static void enqueue_pipeline(lcf_ctx* ctx) {
@@ -903,14 +915,7 @@ static void enqueue_pipeline(lcf_ctx* ctx) {
     }
     stage_event(ctx, ctx->ev[4], s);
     launch_band_order(d, s); L++;
-    L += enqueue_metzger(ctx, true);
-    if (o.method == LCF_METHOD_SVI) launch_svi(d, s);
-    else launch_laplace(d, s);
-    L++;
-    stage_event(ctx, ctx->ev[5], s);
-    launch_refine(d, s); L++;
-    cudaStreamWaitEvent(s, ctx->ev_join_kn, 0);
-    stage_event(ctx, ctx->ev[6], s);
+    L += enqueue_uncertainty(ctx, true);
     if (o.run_multi_bazin && branch == 0) enqueue_mb(s);
     if (branch) cudaStreamWaitEvent(s, ctx->ev_join, 0);
     stage_event(ctx, ctx->ev[7], s);
@@ -1265,16 +1270,7 @@ static void enqueue_finalize(lcf_ctx* ctx, bool given, size_t sel_bytes) {
     cudaEventRecord(ctx->ev[8], s);
     launch_band_order(d, s); L++;
     cudaEventRecord(ctx->ev[4], s);
-    L += enqueue_metzger(ctx, !given);
-    if (!given) {
-        if (ctx->opts.method == LCF_METHOD_SVI) launch_svi(d, s);
-        else launch_laplace(d, s);
-        L++;
-    }
-    cudaEventRecord(ctx->ev[5], s);
-    launch_refine(d, s); L++;
-    cudaStreamWaitEvent(s, ctx->ev_join_kn, 0);
-    cudaEventRecord(ctx->ev[6], s);
+    L += enqueue_uncertainty(ctx, !given);
     cudaEventRecord(ctx->ev[7], s);
     ctx->launches = L;
 }

@@ -293,6 +293,7 @@ struct DeviceBatch {
     int64_t scratch_per_warp;
     double* scratch64;      // FP64 scratch, 5 values per observation
     float* scratch_svi;     // MetzgerKN SVI scratch, 20 values per observation
+    double* mz_lum;         // MetzgerKN scan luminosities, a slice per SM (metzger_block.cuh)
     double* t0_state;       // per band: t0_min, t0_max, best t0 of the profile search
     int64_t t0_slot_base;   // first PsoResult slot of the t0 search region
     int64_t mb_slot_base;   // first PsoResult slot of the MultiBazin region
@@ -374,6 +375,8 @@ void launch_svi_metzger(const DeviceBatch& d, cudaStream_t s);
 void launch_laplace_metzger(const DeviceBatch& d, cudaStream_t s);
 void launch_refine_metzger(const DeviceBatch& d, cudaStream_t s);
 int finalize_init_attributes();
+int polish_init_attributes();
+int64_t mz_lum_doubles(int num_sms);  // DeviceBatch::mz_lum
 double probe_fp32_tflops(int num_sms);
 // polish.cu: FP64 peaks: out[m] = observation-term evaluations per second of
 // the polish's FP64 cost+gradient term for model m (0..6) at full occupancy,

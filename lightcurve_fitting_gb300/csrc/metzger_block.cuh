@@ -25,9 +25,12 @@ constexpr int MZ_BLOCK = 128;
 
 struct MzTables {
     double row[MZ_NG][3][MZ_SLOTS];   // grid time, neutron fraction, heating rate per mass
-    double lum[MZ_NG][MZ_LANES];      // l_rad of each kept sweep
     double pm[MZ_SLOTS];              // phase_max of each t0
+    // l_rad of each kept sweep, in the block's slice of global memory (L2): in
+    // shared memory the block would fill its SM and run beside no other kernel
+    double (*lum)[MZ_LANES];
 };
+constexpr size_t MZ_LUM = (size_t)MZ_NG * MZ_LANES;  // doubles a block
 
 // One grid row: the terms of metzger_sweep64's step that depend on time alone.
 __device__ __forceinline__ void mz_row(int i, double pm, double& t_day, double& xn, double& heat) {

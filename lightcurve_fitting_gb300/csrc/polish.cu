@@ -723,7 +723,8 @@ __device__ __noinline__ SviDeferred svi_deferred_pass(const float4* obs, const f
 // ms = this sample's MetzgerKN sweep rows (value + 4 derivatives per
 // observation), unused by the other models.  Returns false when the
 // reference skips the sample (MetzgerKN peak rescale outside its clamp).
-// Otherwise lls = the log-likelihood (every lane), dl_tot = lane l's FP32
+// Otherwise lls = lane l's part of the log-likelihood (the caller's
+// warp_sum_d, or svi_sum4 of four samples, gives the total), dl_tot = lane l's FP32
 // total d loglik / d theta_{(l >> 2) & 7} (reduce_scatter8f), dlx = lane l's
 // FP64 part of d loglik / d theta_{l & 7} from the upper limits at or near the
 // reference's CDF floor (svi_deferred_pass), floored = 1 when one of them was
@@ -824,7 +825,7 @@ __device__ __forceinline__ bool svi_sample_loglik(const float4* obs, int n, cons
             floored |= r.floored;
         }
     }
-    lls = warp_sum_d((double)ll.s - (double)ll.c);
+    lls = (double)ll.s - (double)ll.c;
     dl_tot = reduce_scatter8f(dll);
     return true;
 }
@@ -842,6 +843,20 @@ struct SviShared {
     int ok[SVI_SAMPLES];             // 0: the reference skips the sample
     int stop;
 };
+
+// Sums four values over the warp in warp_sum_d's order (the same tree, halved
+// between the lanes at its first two levels): lane l returns the total of
+// v[l >> 3].
+__device__ __forceinline__ double svi_sum4(const double* v) {
+    const int lane = threadIdx.x & 31;
+    const bool b4 = lane & 16, b3 = lane & 8;
+    double a[2];
+#pragma unroll
+    for (int i = 0; i < 2; i++) a[i] = (b4 ? v[2 + i] : v[i]) + __shfl_xor_sync(FULL, b4 ? v[i] : v[2 + i], 16);
+    double r = (b3 ? a[1] : a[0]) + __shfl_xor_sync(FULL, b3 ? a[0] : a[1], 8);
+    for (int k = 4; k; k >>= 1) r += __shfl_xor_sync(FULL, r, k);
+    return r;
+}
 
 template <int W>
 __device__ __forceinline__ void svi_sync() {
@@ -891,59 +906,84 @@ __device__ void svi_band(const DeviceBatch& d, int b, SviShared& sh, MzWarp* mz 
         // clamped to [-6, 2]; ~1e-14 relative): the FP64 exp was the step's
         // costliest remaining FP64 call
         const double sg_j = own ? ff_to(ff_exp(ff_from(ls_j))) : 0.0;
+        // Lane 8 g + j: component j of sample g (W = 1), or of the warp's
+        // sample.  The FP64 pipe charges a warp instruction alike for one lane
+        // and for 32, so the four samples' bookkeeping is one instruction each.
+        const int g = lane >> 3, ks = W == 1 ? g : w;
+        const double eps_j = own ? eps_tab[((size_t)step * SVI_SAMPLES + ks) * 7 + j] : 0.0;
+        const double th_j = mu_j + sg_j * eps_j;
+        const float thf = (float)th_j;
+        double part[4] = {0.0, 0.0, 0.0, 0.0}, dlx = 0.0;
+        float dl = 0.0f;
+        bool ok = true;
+#pragma unroll 1
         for (int k = w; k < SVI_SAMPLES; k += W) {
-            const double* ep = eps_tab + ((size_t)step * SVI_SAMPLES + k) * 7;
-            const double eps_j = own ? ep[j] : 0.0;
-            const double th_j = mu_j + sg_j * eps_j;
+            const int src = W == 1 ? 8 * k : 0;
             float pf[MAXP];
 #pragma unroll
-            for (int q = 0; q < MAXP; q++) pf[q] = q < np ? __shfl_sync(FULL, (float)th_j, q) : 0.0f;
+            for (int q = 0; q < MAXP; q++) pf[q] = q < np ? __shfl_sync(FULL, thf, src + q) : 0.0f;
             if constexpr (M == METZGER)
                 metzger_dual_warp(mz[w], pf, (float)bs.t_last, otimes, n, mscr + (size_t)k * 5 * n);
-            double lls, dlx;
+            double dlx_k, part_k;
             float dl_tot;
             int floored;
-            const bool ok = svi_sample_loglik<M>(obs, n, pf, th_j, mscr + (size_t)k * 5 * n, lls, dl_tot, dlx, floored);
-            if (ok) {
-                // lane j: total d loglik / d theta_j (FP32 terms, plus the FP64
-                // terms of deferred upper limits), then its prior and ELBO terms
-                const double dl_j = (double)__shfl_sync(FULL, dl_tot, (4 * j) & 31) + dlx;
-                double lp_j = 0.0, df = 0.0;
-                if (own) {
-                    const double dd = th_j - pc_j;
-                    const double dq = dd * ipw2_j;
-                    lp_j = -0.5 * dd * dq;
-                    df = dl_j - dq;
-                }
-                const double lp = dot8(lp_j, 1.0);
-                if (lane < 8) {
-                    sh.df[k][j] = df;
-                    sh.dfs[k][j] = df * sg_j;
-                    sh.eps[k][j] = eps_j;
-                }
-                if (lane == 0) sh.e[k] = lls + lp;
+            const bool ok_k = svi_sample_loglik<M>(obs, n, pf, W == 1 ? __shfl_sync(FULL, th_j, src + j) : th_j,
+                                                   mscr + (size_t)k * 5 * n, part_k, dl_tot, dlx_k, floored);
+            if (!ok_k) {  // MetzgerKN only (W = SVI_SAMPLES)
+                ok = false;
+                continue;
             }
-            if (lane == 0) sh.ok[k] = ok;
+            // lane j: total d loglik / d theta_j (FP32 terms, plus the FP64
+            // terms of deferred upper limits)
+            const float dl_k = __shfl_sync(FULL, dl_tot, (4 * j) & 31);
+            if (W != 1 || g == k) {
+                dl = dl_k;
+                dlx = dlx_k;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                if (W == 1 ? i == k : i == 0) part[i] = part_k;
         }
+        if (ok) {
+            const double lls = W == 1 ? svi_sum4(part) : warp_sum_d(part[0]);
+            const double dl_j = (double)dl + dlx;
+            double lp_j = 0.0, df = 0.0;
+            if (own) {
+                const double dd = th_j - pc_j;
+                const double dq = dd * ipw2_j;
+                lp_j = -0.5 * dd * dq;
+                df = dl_j - dq;
+            }
+            const double lp = dot8(lp_j, 1.0);
+            if (W == 1 || lane < 8) {
+                sh.df[ks][j] = df;
+                sh.dfs[ks][j] = df * sg_j;
+                sh.eps[ks][j] = eps_j;
+                if (j == 0) sh.e[ks] = lls + lp;
+            }
+        }
+        if (lane == 0)
+            for (int k = w; k < SVI_SAMPLES; k += W) sh.ok[k] = ok;
         svi_sync<W>();
         if (w != 0) continue;
-        double gmu_j = 0.0, gls_j = 0.0, elbo_sum = 0.0;
+        // the samples' sums in order: lanes 0..7 d/d mu_j, lanes 8..15
+        // d/d log sigma_j, lanes 16..23 the ELBO
+        double acc = 0.0;
 #pragma unroll
         for (int q = 0; q < SVI_SAMPLES; q++) {
             if (!sh.ok[q]) continue;
-            gmu_j += sh.df[q][j];
-            gls_j += sh.dfs[q][j] * sh.eps[q][j];
-            elbo_sum += sh.e[q];
+            const double a = g == 0 ? sh.df[q][j] : g == 1 ? sh.dfs[q][j] : sh.e[q];
+            acc = fma(a, g == 1 ? sh.eps[q][j] : 1.0, acc);
         }
+        const double elbo_sum = __shfl_sync(FULL, acc, 16);
         const double ns = (double)SVI_SAMPLES;
         const double ent = dot8(ls_j, 1.0) + 0.5 * (double)np * ln_2pie;
         final_elbo = elbo_sum / ns + ent;
         // Adam, lane i owns variational parameter i
-        const double gmu_i = __shfl_sync(FULL, gmu_j, lane & 7);
-        const double gls_i = __shfl_sync(FULL, gls_j, (lane - np) & 7);
+        const double g_i = __shfl_sync(FULL, acc, lane < np ? lane : 8 + ((lane - np) & 7));
         double gi = 0.0;
-        if (lane < np) gi = -(gmu_i / ns);
-        else if (lane < 2 * np) gi = -(gls_i / ns + 1.0);
+        if (lane < np) gi = -(g_i / ns);
+        else if (lane < 2 * np) gi = -(g_i / ns + 1.0);
         // a component hit by a floored upper limit's ~1e285 term overflows its
         // second moment to +inf and stops, as in the reference
         if (lane < 2 * np && isfinite(gi)) {
@@ -1020,9 +1060,20 @@ void launch_svi(const DeviceBatch& d, cudaStream_t s) {
     if (d.n_bands <= 4096) svi_kernel<SVI_SAMPLES><<<d.n_bands, SVI_BLOCK, 0, s>>>(d);
     else svi_kernel<1><<<(d.n_bands + SVI_SAMPLES - 1) / SVI_SAMPLES, SVI_BLOCK, 0, s>>>(d);
 }
+// The SVI kernels run beside each other and beside the MetzgerKN refinements,
+// which fill most of an SM's shared memory: all prefer the largest split of
+// the L1 cache, so that no SM has to drain to change it.
+int polish_init_attributes() {
+    const cudaFuncAttribute a = cudaFuncAttributePreferredSharedMemoryCarveout;
+    cudaError_t e = cudaFuncSetAttribute(svi_kernel<1>, a, cudaSharedmemCarveoutMaxShared);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(svi_kernel<SVI_SAMPLES>, a, cudaSharedmemCarveoutMaxShared);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(svi_metzger_kernel, a, cudaSharedmemCarveoutMaxShared);
+    return (int)e;
+}
 void launch_svi_metzger(const DeviceBatch& d, cudaStream_t s) {
     if (d.n_bands == 0) return;
-    svi_metzger_kernel<<<std::min(d.n_bands, 5 * d.num_sms), SVI_BLOCK, 0, s>>>(d);
+    // two blocks an SM leave room for the other models' SVI beside them
+    svi_metzger_kernel<<<std::min(d.n_bands, 2 * d.num_sms), SVI_BLOCK, 0, s>>>(d);
 }
 
 // ---------------------------------------------------------------------------
@@ -1082,7 +1133,7 @@ __device__ void svi_grad_point(const float4* obs, int n, float t_last, const dou
             gls_j += df * sg_j * eps_j;
         }
         const double lp = dot8(lp_j, 1.0);
-        elbo_sum += lls + lp;
+        elbo_sum += warp_sum_d(lls) + lp;
     }
     const double ns = (double)n_samples;
     const double ent = dot8(own ? ls_j : 0.0, 1.0) + 0.5 * (double)np * ln_2pie;
