@@ -630,6 +630,9 @@ static int prepare_layout(lcf_ctx* ctx, int n_sources, int n_bands, int64_t n_ob
                 jmax_nb = std::max(jmax_nb, nwd);
             }
         }
+        // longest first: the last of the persistent blocks' tasks are short
+        auto obs_of = [&](int sidx) { return ctx->h_boff[ctx->h_soff[sidx + 1]] - ctx->h_boff[ctx->h_soff[sidx]]; };
+        std::stable_sort(jsrc.begin(), jsrc.end(), [&](int a, int b) { return obs_of(a) > obs_of(b); });
         ctx->n_joint = (int)jsrc.size();
         ctx->joint_max_obs = jmax_obs;
         ctx->joint_max_d = 7 * jmax_nb;
@@ -643,9 +646,8 @@ static int prepare_layout(lcf_ctx* ctx, int n_sources, int n_bands, int64_t n_ob
             rc2 |= grow(ctx, ctx->joint_src, jsrc.size() * sizeof(int32_t));
             rc2 |= grow(ctx, ctx->joint_res, jsrc.size() * 3 * sizeof(JointResult));
             // the persistent swarm's grid and its blocks' state
-            ctx->joint_grid = joint_grid(jmax_obs, ctx->joint_max_d, ctx->num_sms);
-            rc2 |= grow(ctx, ctx->joint_state,
-                        (size_t)ctx->joint_grid * JOINT_STATE_ARRAYS * ctx->joint_max_d * 200 * sizeof(float));
+            ctx->joint_grid = joint_grid(ctx->n_joint, jmax_obs, ctx->joint_max_d, ctx->num_sms);
+            rc2 |= grow(ctx, ctx->joint_state, joint_state_bytes(ctx->joint_grid, ctx->joint_max_d));
             // draws per seed: init (2 D P) + 1500 iterations x 2 D P
             int64_t need = (int64_t)3002 * ctx->joint_max_d * 200;
             int64_t need_init = (int64_t)2 * ctx->joint_max_d * 200;

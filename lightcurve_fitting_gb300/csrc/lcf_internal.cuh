@@ -34,9 +34,6 @@ constexpr double SVI_LR = 0.01;
 // 42 joint parameters.
 constexpr int J_MAX_BANDS = 6;
 constexpr int J_MAX_D = 7 * J_MAX_BANDS;
-// Per-particle arrays of the joint swarm's state: position, velocity and
-// personal best as double-float pairs, and the trial position.
-constexpr int JOINT_STATE_ARRAYS = 7;
 
 __host__ __device__ constexpr int n_params_of(int m) {
     return m == BAZIN ? 6 : m == VILLAR ? 7 : m == TDE ? 7 : m == ARNETT ? 5 : m == MAGNETAR ? 5 : m == SHOCK ? 5
@@ -309,8 +306,8 @@ struct DeviceBatch {
     const double* joint_draws64;  // [3][joint_init_per_seed] the first uniforms (initialisation) in FP64
     int64_t joint_draws_per_seed;
     int64_t joint_init_per_seed;
-    float* joint_state;          // [joint_grid][JOINT_STATE_ARRAYS][joint_max_d][200] swarm state
-    int joint_grid;              // blocks of the persistent joint swarm
+    float* joint_state;          // the swarm state of the joint_grid teams (joint_state_bytes)
+    int joint_grid;              // teams of the persistent joint swarm
     int joint_max_obs;           // most observations of a joint source
     int joint_max_d;             // most joint parameters of a joint source
 };
@@ -390,6 +387,7 @@ void launch_band_cost(int model, const float4* obs, int n, float t_last, const d
 // Host-side generation of the RNG tables (host.cpp)
 void make_draw_tables(float* draws, double* draws64, float2* draws15, double* svi_eps);
 void make_joint_draws(float2* draws15, double* draws64, int64_t per_seed, int64_t init_per_seed);
-int joint_grid(int max_obs, int max_d, int num_sms);
+size_t joint_state_bytes(int grid, int max_d);
+int joint_grid(int n_joint, int max_obs, int max_d, int num_sms);
 
 }  // namespace lcf
