@@ -9,8 +9,9 @@
 //     fit (:1008-1157), whose PSO runs execute in pso.cu and whose task lists
 //     are appended here on the device, so the whole sequence needs no host
 //     round trip.
-// One warp per band; the lanes split the observations, the FP64 sums are
-// reduced across the warp.
+// One warp per band, the lanes splitting the observations and the FP64 sums
+// reduced across the warp; MetzgerKN, whose light curve is a sequential
+// integration, takes a block per band with an integration a lane.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -28,10 +29,6 @@ __device__ __forceinline__ double wsum(double v) {
     for (int k = 16; k; k >>= 1) v += __shfl_xor_sync(FULL, v, k);
     return v;
 }
-__device__ __forceinline__ double wmax(double v) {
-    for (int k = 16; k; k >>= 1) v = fmax(v, __shfl_xor_sync(FULL, v, k));
-    return v;
-}
 
 struct BandView {
     const double *t, *f, *fe, *var, *uf, *mag;
@@ -47,49 +44,18 @@ __device__ __forceinline__ BandView band_view(const DeviceBatch& d, const BandSt
     return v;
 }
 
-// Prediction of observation i (lanes call with their own i).  For MetzgerKN
-// the whole band is first evaluated by lane 0 into `scr` (the sweep is
-// sequential over the grid).
-struct Predictor {
-    int m;
-    const double* p;
-    const double* scr;
+// neg_log_posterior, src/parametric.rs:2464-2511 (models other than
+// MetzgerKN).  Out of line: called for one value and, rarely, for a stencil,
+// and inlined it would change how the Hessian's own products are contracted.
+__device__ __noinline__ double neg_log_posterior_w(int m, const BandView& b, const double* p) {
+    int lane = threadIdx.x & 31;
     Model64 mod;
-    __device__ Predictor(int m_, const double* p_, const double* s_) : m(m_), p(p_), scr(s_) {
-        if (m != 7) mod.init(m, p);
-    }
-    __device__ double operator()(const BandView& b, int i) const {
-        return m == 7 ? scr[i] : mod.eval(b.t[i], nullptr);
-    }
-};
-__device__ void metzger_prepare(int m, const double* p, const BandView& b, double* scr) {
-    if (m != 7) return;
-    if ((threadIdx.x & 31) == 0) metzger_f64(p, b.t, b.n, scr);
-    __syncwarp();
-}
-
-// MetzgerKN rescale of the non-upper peak to 1 (src/parametric.rs:1325-1337)
-__device__ double metzger_scale(const Predictor& P, const BandView& b) {
-    int lane = threadIdx.x & 31;
-    double mx = -INFINITY;
-    for (int i = lane; i < b.n; i += 32)
-        if (!b.up[i]) mx = fmax(mx, P(b, i));
-    mx = wmax(mx);
-    if (mx > 1e-10 && isfinite(mx)) return fmin(fmax(1.0 / mx, 0.1), 10.0);
-    return 1.0;
-}
-
-// neg_log_posterior, src/parametric.rs:2464-2511
-__device__ double neg_log_posterior_w(int m, const BandView& b, const double* p, double* scr) {
-    int lane = threadIdx.x & 31;
-    metzger_prepare(m, p, b, scr);
-    Predictor P(m, p, scr);
-    double scale = m == 7 ? metzger_scale(P, b) : 1.0;
+    mod.init(m, p);
     double se2 = exp(2.0 * p[se_idx_of(m)]);
     double nll = 0.0;
     int nonfinite = 0;
     for (int i = lane; i < b.n; i += 32) {
-        double pr = P(b, i) * scale;
+        double pr = mod.eval(b.t[i], nullptr);
         if (!isfinite(pr)) { nonfinite = 1; continue; }
         double tv = b.var[i] + se2;
         if (b.up[i]) nll -= log_normal_cdf_f64((b.uf[i] - pr) / sqrt(tv));
@@ -107,30 +73,6 @@ __device__ double neg_log_posterior_w(int m, const BandView& b, const double* p,
     }
     __syncwarp();
     return nll + nlp;
-}
-
-// Band log-likelihood skipping non-finite predictions (the profile scans,
-// src/parametric.rs:2716-2726, :2916-2932)
-__device__ double band_ll_w(int m, const BandView& b, const double* p, double* scr, bool metzger_rescale) {
-    int lane = threadIdx.x & 31;
-    metzger_prepare(m, p, b, scr);
-    Predictor P(m, p, scr);
-    double scale = (m == 7 && metzger_rescale) ? metzger_scale(P, b) : 1.0;
-    double se2 = exp(2.0 * p[se_idx_of(m)]);
-    double ll = 0.0;
-    for (int i = lane; i < b.n; i += 32) {
-        double pr = P(b, i) * scale;
-        if (!isfinite(pr)) continue;
-        double tv = b.var[i] + se2;
-        if (b.up[i]) ll += log_normal_cdf_f64((b.uf[i] - pr) / sqrt(tv));
-        else {
-            double r = b.f[i] - pr;
-            ll += -0.5 * (r * r / tv + log(2.0 * 3.14159265358979323846 * tv));
-        }
-    }
-    ll = wsum(ll);
-    __syncwarp();
-    return ll;
 }
 
 // ---------------------------------------------------------------------------
@@ -187,7 +129,8 @@ __device__ double ll_scan_t(const double* p, const float4* obs, const BandView& 
     return wsum(ll);
 }
 
-// band_ll_w for the models other than MetzgerKN, FP32 evaluation
+// Band log-likelihood skipping non-finite predictions (the profile scans,
+// src/parametric.rs:2716-2726, :2916-2932), models other than MetzgerKN
 __device__ double band_ll_fast(int m, const double* p, const float4* obs, const BandView& b, const double* cst) {
     switch (m) {
         case BAZIN: return ll_scan_t<BazinF>(p, obs, b, cst);
@@ -261,7 +204,7 @@ struct MzLl {
     }
 };
 
-// band_ll_w for MetzgerKN by one lane (rescale: the PSO cost's peak rescale)
+// The same for MetzgerKN by one lane (rescale: the PSO cost's peak rescale)
 __device__ double metzger_ll_lane(MzTables& T, int slot, int col, const double* p, const BandView& b,
                                   const double* cst, bool rescale) {
     int j_start = b.n;
@@ -743,7 +686,6 @@ __global__ void laplace_kernel(DeviceBatch d) {
     if (!bs.valid || o.model < 0 || o.model == METZGER) return;
     BandView b = band_view(d, bs);
     int m = o.model, nf = n_params_of(m), se = se_idx_of(m);
-    double* scr = d.scratch64 + 5 * bs.off;
     double mp[MAXP];
     for (int j = 0; j < nf; j++) mp[j] = o.pso_params[j];
     int idx[MAXP], ns = 0;
@@ -752,7 +694,7 @@ __global__ void laplace_kernel(DeviceBatch d) {
     double H[36];
     // the analytic Hessian (forward over the adjoint); points with non-finite
     // predictions keep the reference's central differences
-    const double f0 = neg_log_posterior_w(m, b, mp, scr);
+    const double f0 = neg_log_posterior_w(m, b, mp);
     const bool analytic = f0 < 1e99 && laplace_hessian_analytic(m, b, mp, idx, ns, H);
     for (int si = 0; si < ns && !analytic; si++) {
         int i = idx[si];
@@ -767,7 +709,7 @@ __global__ void laplace_kernel(DeviceBatch d) {
                 for (int t = 0; t < nf; t++) q[t] = mp[t];
                 q[i] += si_[k] * hi;
                 q[j] += sj_[k] * hj;
-                fv[k] = neg_log_posterior_w(m, b, q, scr);
+                fv[k] = neg_log_posterior_w(m, b, q);
             }
             double h = (fv[0] - fv[1] - fv[2] + fv[3]) / (4.0 * hi * hj);
             H[si * ns + sj] = h;
@@ -967,9 +909,10 @@ __global__ void refine_kernel(DeviceBatch d) {
     double msum = 0.0;
     int mcount = 0;
     {
-        Predictor P(m, mu, scr);
+        Model64 P;
+        P.init(m, mu);
         int npos = 0;
-        for (int i = lane; i < b.n; i += 32) npos += (P(b, i) * b.peak > 0.0) ? 1 : 0;
+        for (int i = lane; i < b.n; i += 32) npos += (P.eval(b.t[i], nullptr) * b.peak > 0.0) ? 1 : 0;
         for (int k = 16; k; k >>= 1) npos += __shfl_xor_sync(FULL, npos, k);
         __syncwarp();
         const double* use = mu;
@@ -979,9 +922,10 @@ __global__ void refine_kernel(DeviceBatch d) {
             for (int j = 0; j < np; j++) pso[j] = o.pso_params[j];
             use = pso;
         }
-        Predictor Q(m, use, scr);
+        Model64 Q;
+        Q.init(m, use);
         for (int i = lane; i < b.n; i += 32) {
-            double pf = Q(b, i) * b.peak;
+            double pf = Q.eval(b.t[i], nullptr) * b.peak;
             if (pf > 0.0 && b.f[i] > 0.0) {
                 double mpred = -2.5 * log10(pf) + 23.9;
                 double merr = 1.0857 * b.fe[i] / b.f[i];

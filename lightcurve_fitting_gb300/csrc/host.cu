@@ -1,18 +1,19 @@
 // host.cu — context, device memory, the stage sequence of the fused fit,
 // CUDA-graph capture, and the C ABI of include/lcf.h.
 //
-// Stage sequence of one fit (all on the context's stream, captured once per
-// batch layout into a CUDA graph and replayed):
+// Stage sequence of one fit (captured once per batch layout into a CUDA graph
+// and replayed; on the context's stream but for the two forks):
 //   prep          normalise bands, FP32 records, stats, rank inside source
 //   pso[0]        3 restarts x 8 models per band + MultiBazin K = 1
 //   lbfgs         best restart + bounded L-BFGS per (band, model)
 //   select        BIC model selection
 //   (gate)        fit_all_models == false: Bazin first, the 7 others only
 //                 for bands whose Bazin cost is >= 2 (device-built tasks)
+//   (joint)       the joint multi-band swarms of sources with >= 2 bands
 //   t0 search     SVI mode, rank-0 bands: 5 coarse + 3 fine PSO runs
-//   svi | laplace
-//   refine        profile t0 + all-parameter refinement + mag chi2
-//   MultiBazin    K = 2, 3, 4 (device-built tasks, early stop)
+//   svi | laplace, then refine (profile t0 + all-parameter refinement + mag
+//                 chi2): the MetzgerKN bands, the others on a second stream
+//   MultiBazin    K = 2, 3, 4 (device-built tasks, early stop), on a third
 #include <cuda_runtime.h>
 
 #include <algorithm>

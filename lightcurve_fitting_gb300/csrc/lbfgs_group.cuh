@@ -27,10 +27,9 @@
 //
 // The polish is bound by instruction fetch (its double-float terms and FP64
 // line search are long code; measured on GB300, more resident warps at
-// different points of it made it slower, and a warp on its own spends ~15 us
-// on an observation's term).  The warps of a block run a round in step: a
-// block barrier before and after the evaluation, so that they fetch the same
-// code.  On small batches too: 1,000 uneven sources polish in 79 ms in step
+// different points of it made it slower).  The warps of a block run a round
+// in step: a block barrier before and after the evaluation, so that they
+// fetch the same code.  On small batches too: 1,000 uneven sources polish in 79 ms in step
 // and in 96 ms without the barriers.  The group's scalar state and the per-lane
 // vectors live in shared memory, leaving the registers to the evaluation.
 //

@@ -73,7 +73,8 @@ __global__ void __launch_bounds__(LCF_LB_BLOCK, LCF_LB_MINB)
             case MAGNETAR: polish_model<MAGNETAR>(d, w, n_long, n_mid); break;
             case SHOCK: polish_model<SHOCK>(d, w, n_long, n_mid); break;
             case AFTERGLOW: polish_model<AFTERGLOW>(d, w, n_long, n_mid); break;
-            default: polish_model<METZGER>(d, w, n_long, n_mid); break;
+            // MetzgerKN keeps its swarm's result: the queue only chooses the restart
+            default: polish_queue<METZGER, 8, 8>(d, w, 0, d.n_bands, &d.ctr->lb_next[METZGER]); break;
         }
     }
 }

@@ -2,9 +2,11 @@
 //
 // One warp runs one swarm (a PSO task: band x model x restart, a profile-t0
 // run, or a MultiBazin run); lane p holds particle p (30 of 32 lanes).  The
-// band's observations are staged once per task into the warp's slice of
-// shared memory with a TMA bulk copy and read by all lanes at the same index
-// (broadcast), so the inner loop touches no HBM.
+// longest swarms of a batch, whose ends the launch would wait for, are run by
+// a block: its first warp moves the particles, and all warps evaluate them
+// (run_team).  The band's observations are staged once per task into the
+// warp's slice of shared memory with a TMA bulk copy and read by all lanes at
+// the same index (broadcast), so the inner loop touches no HBM.
 //
 // The reference updates the global best *inside* its particle loop
 // (pso_minimize, src/parametric.rs:1698-1741): particle p moves towards the
