@@ -229,7 +229,7 @@ struct Counters {
     unsigned long long lb_obs_evals_by_model[8];  // observation x (cost + gradient) evaluations, by model
     unsigned long long lb_fp64_obs_evals_by_model[8];  // of which in FP64 (ff range fallback)
     int32_t sort_hist[8][256];  // per slot: key histogram, then offsets, of the device task sort
-    int32_t band_hist[16];      // bands by selected model, in band_order's grouping (0: MetzgerKN)
+    int32_t band_hist[16];      // 0: the MetzgerKN bands, band_order's first
     int32_t polish_hist[256];   // bands by length: histogram, then offsets (polish_order)
     int32_t lb_next[8];         // per model: next index of the polish queue (eight lanes a band)
     int32_t lb_next_long[8];    // per model: next index of its long bands (a warp a band)
@@ -363,7 +363,9 @@ int launch_joint(const DeviceBatch& d, cudaStream_t s);
 size_t joint_smem_bytes(int max_obs, int max_d);
 // finalize.cu
 void launch_laplace(const DeviceBatch& d, cudaStream_t s);
-// bands grouped by selected model into d.band_order, their counts into ctr->band_hist
+// SVI gives every band of a batch of so few bands four warps (launch_svi)
+inline bool svi_wide(int n_bands) { return n_bands <= 4096; }
+// bands by selected model and length into d.band_order, the number of MetzgerKN ones into ctr->band_hist[0]
 void launch_band_order(const DeviceBatch& d, cudaStream_t s);
 void launch_refine(const DeviceBatch& d, cudaStream_t s);
 // the MetzgerKN bands of SVI, Laplace and the refinements, which the kernels

@@ -1058,7 +1058,7 @@ __global__ void __launch_bounds__(SVI_BLOCK) svi_metzger_kernel(DeviceBatch d) {
 // bound by throughput and runs a warp a band (10,000 sources: 175 / 203 ms).
 void launch_svi(const DeviceBatch& d, cudaStream_t s) {
     if (d.n_bands == 0) return;
-    if (d.n_bands <= 4096) svi_kernel<SVI_SAMPLES><<<d.n_bands, SVI_BLOCK, 0, s>>>(d);
+    if (svi_wide(d.n_bands)) svi_kernel<SVI_SAMPLES><<<d.n_bands, SVI_BLOCK, 0, s>>>(d);
     else svi_kernel<1><<<(d.n_bands + SVI_SAMPLES - 1) / SVI_SAMPLES, SVI_BLOCK, 0, s>>>(d);
 }
 // The SVI kernels run beside each other and beside the MetzgerKN refinements,
