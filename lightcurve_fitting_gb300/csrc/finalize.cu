@@ -512,9 +512,10 @@ __device__ void jacobi_eigen(double* a, int n, double* ev, double* V) {
 //     together (10,000 uneven sources, SVI 178 -> 162 ms, refinements 41 -> 28
 //     against bands of a model in any order; longest first over all models
 //     221 and 59).
-//   - A smaller one (svi_wide) waits for its longest bands: they come first, in
-//     classes of 64 observations over all models (1,000 sources, SVI 43 -> 38
-//     ms, against 43 model by model).
+//   - One of up to 4,096 bands waits for its longest bands: they come first, in
+//     classes of 64 observations over all models (1,000 sources, SVI 38 ms
+//     against 43 model by model, 2,400 given pairs 33 against 37 in all).  At
+//     9,000 bands SVI is 60 against 68 ms, but the refinements 20 against 12.
 // ---------------------------------------------------------------------------
 constexpr int BO_LEN = 64, BO_KEYS = 9 * BO_LEN;
 __device__ __forceinline__ int band_order_key(const DeviceBatch& d, int b, bool by_length) {
@@ -557,7 +558,7 @@ __global__ void __launch_bounds__(BO_BLOCK) band_order_kernel(DeviceBatch d, boo
 }
 void launch_band_order(const DeviceBatch& d, cudaStream_t s) {
     if (d.n_bands == 0) return;
-    band_order_kernel<<<1, BO_BLOCK, 0, s>>>(d, svi_wide(d.n_bands));
+    band_order_kernel<<<1, BO_BLOCK, 0, s>>>(d, d.n_bands <= 4096);
 }
 
 // neg_log_posterior (src/parametric.rs:2464-2511) of MetzgerKN at one

@@ -750,6 +750,7 @@ static int prepare_layout(lcf_ctx* ctx, int n_sources, int n_bands, int64_t n_ob
     d.n_sources = n_sources;
     d.n_bands = n_bands;
     d.num_sms = ctx->num_sms;
+    d.svi_wide = svi_wide(n_bands, o.fit_all_models);
     d.n_obs = n_obs;
     d.stats = (BandStats*)ctx->stats_b.p;
     d.obs = (float4*)ctx->obs.p;

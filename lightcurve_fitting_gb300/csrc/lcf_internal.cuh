@@ -247,6 +247,7 @@ struct DeviceBatch {
     const int32_t* src_off;
     int n_sources, n_bands;
     int num_sms;
+    int svi_wide;                // SVI with four warps a band (launch_svi)
     int64_t n_obs;
     // prepared
     BandStats* stats;
@@ -363,8 +364,6 @@ int launch_joint(const DeviceBatch& d, cudaStream_t s);
 size_t joint_smem_bytes(int max_obs, int max_d);
 // finalize.cu
 void launch_laplace(const DeviceBatch& d, cudaStream_t s);
-// SVI gives every band of a batch of so few bands four warps (launch_svi)
-inline bool svi_wide(int n_bands) { return n_bands <= 4096; }
 // bands by selected model and length into d.band_order, the number of MetzgerKN ones into ctr->band_hist[0]
 void launch_band_order(const DeviceBatch& d, cudaStream_t s);
 void launch_refine(const DeviceBatch& d, cudaStream_t s);
@@ -373,6 +372,7 @@ void launch_refine(const DeviceBatch& d, cudaStream_t s);
 void launch_svi_metzger(const DeviceBatch& d, cudaStream_t s);
 void launch_laplace_metzger(const DeviceBatch& d, cudaStream_t s);
 void launch_refine_metzger(const DeviceBatch& d, cudaStream_t s);
+bool svi_wide(int n_bands, bool all_models);
 int finalize_init_attributes();
 int polish_init_attributes();
 int64_t mz_lum_doubles(int num_sms);  // DeviceBatch::mz_lum

@@ -1053,12 +1053,18 @@ __global__ void __launch_bounds__(SVI_BLOCK) svi_metzger_kernel(DeviceBatch d) {
 }
 
 // The 1000-step chain bounds a batch that does not keep the chip's warp slots
-// filled: four warps a band then shorten it (1,000 uneven sources with a warp
-// / four warps a band: 62 / 42 ms, one source 3.2 / 1.7).  A larger batch is
-// bound by throughput and runs a warp a band (10,000 sources: 175 / 203 ms).
+// filled: four warps a band then shorten it.  A larger batch is bound by
+// throughput and runs a warp a band.  SVI + refinements, ms, a warp / four
+// warps a band, of fits over all models: one source 3.8 / 2.2, 1,000 (3,000
+// bands) 69 / 44, 2,000 86 / 60, 3,000 101 / 80, 4,500 118 / 103, 6,500
+// 139 / 147, 10,000 193 / 243.  Given pairs, an eighth of them MetzgerKN whose
+// kernels fill the slots beside, and the bands of one model change over
+// earlier: 2,400 pairs 43 / 32, 4,800 59 / 58, 9,600 91 / 105; the joint fit's
+// 4,500 bands 47 / 48, 7,500 73 / 79.
+bool svi_wide(int n_bands, bool all_models) { return n_bands <= (all_models ? 12288 : 4096); }
 void launch_svi(const DeviceBatch& d, cudaStream_t s) {
     if (d.n_bands == 0) return;
-    if (svi_wide(d.n_bands)) svi_kernel<SVI_SAMPLES><<<d.n_bands, SVI_BLOCK, 0, s>>>(d);
+    if (d.svi_wide) svi_kernel<SVI_SAMPLES><<<d.n_bands, SVI_BLOCK, 0, s>>>(d);
     else svi_kernel<1><<<(d.n_bands + SVI_SAMPLES - 1) / SVI_SAMPLES, SVI_BLOCK, 0, s>>>(d);
 }
 // The SVI kernels run beside each other and beside the MetzgerKN refinements,
