@@ -43,6 +43,7 @@ constexpr int J_MAXIT = 1500;
 constexpr int J_STALL = 60;
 constexpr int J_THREADS = 448;   // of a block
 constexpr int J_WARPS = J_THREADS / 32;
+
 // de Soto et al. relative priors of the offsets, src/parametric.rs:3771-3786
 static __device__ __constant__ float c_rel_mean[7] = {-0.015f * 2.302585093f, -0.001f, -0.095f * 2.302585093f,
                                                       -1.181f, -0.195f * 2.302585093f, -0.323f * 2.302585093f,
@@ -259,8 +260,8 @@ static __host__ __device__ size_t joint_state_floats(int max_d) { return (size_t
 //   - the next iteration's draws are asked into L2 early (2 %);
 //   - a lone task is spread over a cluster of four blocks, each with every
 //     fourth particle, whose rounds meet in two cluster barriers.
-// 100 basic sources (3 x 30): 44.2 -> 29.0 ms; 500 uneven ones: 145 -> 103;
-// 20 long ones (3 x 1000): 378 -> 126 (this kernel's stage).
+// This stage of 100 basic sources (3 x 30): 44 -> 31 ms; of 500 uneven ones:
+// 145 -> 103; the whole fit of 20 long ones (3 x 1000): 442 -> 189.
 template <int C, int PER_SM>
 __global__ void __launch_bounds__(J_THREADS, PER_SM) joint_pso_kernel(DeviceBatch d) {
     using Team = JointTeam<C>;
