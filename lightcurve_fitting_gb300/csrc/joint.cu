@@ -96,7 +96,7 @@ __device__ double joint_cost(const JointBands& jb, const float4* obs, const floa
 #pragma unroll
         for (int j = 0; j < 7; j++) ref[j] = 0.0f;
     {
-        float c = VillarF::constraint(ref);
+        float c = VillarF::constraint_swarm(ref);
         if (open && c > 0.0f) { cost = 1e12 + 10000.0 * (double)c; open = false; }
     }
     // the band sums as double-float pairs: ~1e-14 relative, far below the FP32
@@ -108,7 +108,7 @@ __device__ double joint_cost(const JointBands& jb, const float4* obs, const floa
 #pragma unroll
         for (int j = 0; j < 7; j++) bp[j] = b == 0 || !live ? ref[j] : ref[j] + xs[(7 * b + j) * JP + p].x;
         if (b > 0) {
-            float c = VillarF::constraint(bp);
+            float c = VillarF::constraint_swarm(bp);
             if (open && c > 0.0f) { cost = 1e12 + 10000.0 * (double)c; open = false; }
         }
         if (!__any_sync(FULL, open)) break;
