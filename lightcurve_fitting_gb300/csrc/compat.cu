@@ -376,7 +376,7 @@ __device__ __noinline__ void svi_source(const SviArgs& A, int s, int o0, int o1,
                         exp(-a * a);
                     const double lc = z < -30.0 ? -0.5 * z * z - 0.5 * log(2.0 * PI) - log(-z)
                                                 : log(fmax(z > 0.0 ? 1.0 - 0.5 * e2 : 0.5 * e2, 1e-300));
-                    if (z <= 8.0) v[0] += lc;
+                    if (!(z > 8.0)) v[0] += lc;  // NaN: ln 1e-300, as log_normal_cdf_f64 has it
                     const double erf = z >= 0.0 ? 1.0 - e2 : -(1.0 - e2);
                     const double phi = exp(-0.5 * z * z) * 0.39894228040143267794;
                     const double ratio = phi / fmax(0.5 * (1.0 + erf), 1e-300);
