@@ -102,8 +102,11 @@ __device__ __forceinline__ bool mz_sweep(MzTables& T, const double* p, int slot,
 __device__ __forceinline__ double mz_interp(const MzTables& T, int slot, int col, double ph, int& i) {
     while (i < MZ_NG && ph > T.row[i][0][slot]) i++;
     if (i == MZ_NG) return T.lum[MZ_NG - 1][col];
+    if (i == 0) {
+        if (ph <= T.row[0][0][slot]) return T.lum[0][col];
+        i = 1;  // a NaN phase: NaN from the first interval, as in metzger_sweep64
+    }
     const double l_rad = T.lum[i][col];
-    if (i == 0) return l_rad;
     const double prev_t = T.row[i - 1][0][slot], prev_l = T.lum[i - 1][col];
     double frac = (ph - prev_t) / (T.row[i][0][slot] - prev_t);
     return prev_l + frac * (l_rad - prev_l);

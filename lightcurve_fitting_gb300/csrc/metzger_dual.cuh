@@ -355,11 +355,12 @@ __device__ __forceinline__ void metzger_dual_warp(MzWarp& W, const float* pv, fl
     for (int j = lane >> 2; j < n; j += 8) {
         D l(0.0f);
         const float phv = t(j) - pv[3];
-        if (ok && phv > 0.0f) {
-            // the first grid point not before the phase
+        if (ok && !(phv <= 0.0f)) {
+            // the first grid point not before the phase (a NaN phase: NaN from the first interval)
             int i = 0;
             for (int step = 128; step; step >>= 1)
                 if (i + step <= 200 && phv > W.row[i + step - 1][0]) i += step;
+            if (i == 0 && !(phv <= W.row[0][0])) i = 1;
             if (i == 0 || i == 200) {
                 const int g = i == 0 ? 0 : 199;
                 l.v = W.lum[g][0];
