@@ -1,6 +1,6 @@
 // metzger_dual.cuh — MetzgerKN prediction and its derivatives with respect to
 // (log10 M_ej, log10 v_ej, log10 kappa, t0) by forward-mode differentiation in
-// FP32 (dual numbers with four tangents).
+// FP32 (dual numbers).
 //
 // The reference differentiates MetzgerKN for SVI by forward differences of
 // its FP64 model with step 1e-5 (metzger_kn_grad_batch_into,
@@ -86,151 +86,19 @@ __device__ __forceinline__ DN<K> dpowc(const DN<K>& a, float c) {  // a^c, a > 0
 template <int K>
 __device__ __forceinline__ DN<K> datan(const DN<K>& a) { return mk(atanf(a.v), 1.0f / (1.0f + a.v * a.v), a); }
 
-// The sweep with the tangents of parameters tan0 .. tan0 + K - 1 (of
-// log10 M_ej, log10 v_ej, log10 kappa, t0): writes, for the sorted
-// observation times `t[j]`, the unnormalised interpolant to out[j * 5] and
-// its tangents to out[j * 5 + 1 + tan0 + k]; lp_v / lp_d receive the peak
-// and its tangents.  Returns false when the reference returns all zeros
-// (phase_max <= 0.01, or a non-positive or non-finite peak).  The same
-// arithmetic for every K: instances with fewer tangents (one parameter per
-// lane) split the work of the four-tangent sweep across lanes.
-template <int K, class Times>
-__device__ bool metzger_dual_raw(const float* pv, int tan0, float t_last, const Times& t, int n, float* out,
-                                 float& lp_v, float* lp_d) {
-    using D = DN<K>;
-    const float MSUN30 = 1.989e3f, C = 2.998e10f, SPD = 86400.0f, PI_F = 3.14159265358979f, LN10F = 2.302585093f;
-    D p0(pv[0]), p1(pv[1]), p2(pv[2]), t0(pv[3]);
-#pragma unroll
-    for (int k = 0; k < K; k++) {
-        const int q = tan0 + k;
-        if (q == 0) p0.d[k] = 1.0f;
-        if (q == 1) p1.d[k] = 1.0f;
-        if (q == 2) p2.d[k] = 1.0f;
-        if (q == 3) t0.d[k] = 1.0f;
-    }
-    D m30 = dexp(p0 * LN10F) * MSUN30;
-    D v = dexp(p1 * LN10F) * C;
-    D kappa_r = dexp(p2 * LN10F);
-    float pm = t_last - t0.v;
-    for (int j = 0; j < n; j++) {
-        out[j * 5] = 0.0f;
-#pragma unroll
-        for (int k = 0; k < K; k++) out[j * 5 + 1 + tan0 + k] = 0.0f;
-    }
-    lp_v = 0.0f;
-#pragma unroll
-    for (int k = 0; k < K; k++) lp_d[k] = 0.0f;
-    if (!(pm > 0.01f)) return false;
-    D phase_max = (t0 * -1.0f) + t_last;
-    const float lmin = -4.605170185988091f;
-    D lmax = dlog(phase_max * 1.05f);
-    D dl = (lmax - lmin) * (1.0f / 199.0f);
-    const float xn0 = 0.8f, xr = 0.2f;
-    D vs = v * 1e-5f;
-    D e_th = m30 * vs * vs * 0.5f;
-    D e_kin = e_th;
-    D t_day = D(0.01f);
-    D r = t_day * v * SPD;
-    D mos = m30 * 1e-10f;
-    D diff_k = m30 * (3.0f / (4.0f * PI_F * C) * 1e30f);
-    D l_peak = D(-INFINITY);
-    D prev_t = t_day, prev_l = D(0.0f);
-    int j = 0;
-    while (j < n && t(j) - t0.v <= 0.0f) j++;  // zeros already written
-    for (int i = 0; i < 200; i++) {
-        D t_next = dexp(dl * (float)(i + 1) + lmin);
-        D t_sec = t_day * SPD;
-        D ef = dpowc(t_day, 0.74f) * 0.34f;
-        D eth = (dexp(t_day * -0.56f) + (ef.v > 1e-10f ? dlog1p(ef) / ef : D(1.0f))) * 0.36f;
-        D xn = dexp(t_sec * (-1.0f / 900.0f)) * xn0;
-        D tt = datan(D(0.11f) / (t_sec - 1.3f)) * (1.0f / PI_F);
-        if (tt.v < 1e-30f) tt = D(1e-30f);
-        D eps_rp = eth * dpowc(tt, 1.3f) * 2e18f;
-        D l_heat = mos * (xn * 3.2e14f + eps_rp);
-        D kappa_eff = (D(xn0) - xn) * 0.4f + kappa_r * xr;
-        D t_diff = kappa_eff * diff_k / (v * t_sec) + r * (1.0f / C);
-        D l_rad = (e_th.v > 0.0f && t_diff.v > 0.0f) ? e_th / t_diff : D(0.0f);
-        if (l_rad.v > l_peak.v) l_peak = l_rad;
-        if (i == 0) {
-            while (j < n && t(j) - t0.v <= t_day.v) {
-                out[j * 5] = l_rad.v;
-#pragma unroll
-                for (int k = 0; k < K; k++) out[j * 5 + 1 + tan0 + k] = l_rad.d[k];
-                j++;
-            }
-        } else {
-            while (j < n) {
-                float phv = t(j) - t0.v;
-                if (phv > t_day.v) break;
-                D ph = (t0 * -1.0f) + t(j);
-                D lv = prev_l + (ph - prev_t) / (t_day - prev_t) * (l_rad - prev_l);
-                out[j * 5] = lv.v;
-#pragma unroll
-                for (int k = 0; k < K; k++) out[j * 5 + 1 + tan0 + k] = lv.d[k];
-                j++;
-            }
-        }
-        prev_t = t_day;
-        prev_l = l_rad;
-        D l_pdv = r.v > 0.0f ? e_th * v / r : D(0.0f);
-        if (i < 199) {
-            D dts = (t_next - t_day) * SPD;
-            e_th = e_th + (l_heat - l_pdv - l_rad) * dts;
-            if (e_th.v < 0.0f) e_th = D(0.0f);
-            e_kin = e_kin + l_pdv * dts;
-            D vn = dsqrt(e_kin * 2.0f / mos);
-            v = vn.v < C ? vn : D(C);
-            r = r + v * dts;
-        }
-        t_day = t_next;
-    }
-    while (j < n) {
-        out[j * 5] = prev_l.v;
-#pragma unroll
-        for (int k = 0; k < K; k++) out[j * 5 + 1 + tan0 + k] = prev_l.d[k];
-        j++;
-    }
-    lp_v = l_peak.v;
-#pragma unroll
-    for (int k = 0; k < K; k++) lp_d[k] = l_peak.d[k];
-    return l_peak.v > 0.0f && isfinite(l_peak.v);
-}
-
-// Writes, for the sorted observation times `t[j]` (stride 1), the normalised
-// prediction and its four derivatives to out[j * 5 + {0..4}].  Returns false
-// when the reference returns all zeros (phase_max <= 0.01, or a non-positive
-// or non-finite peak); out is then zero.
-template <class Times>
-__device__ bool metzger_dual_sweep(const float* pv, float t_last, const Times& t, int n, float* out) {
-    float lp_v, lp_d[4];
-    if (!metzger_dual_raw<4>(pv, 0, t_last, t, n, out, lp_v, lp_d)) {
-        for (int q = 0; q < n * 5; q++) out[q] = 0.0f;
-        return false;
-    }
-    // normalise by the peak (its tangent included, as the difference quotient has it)
-    float ip = 1.0f / lp_v;
-    for (int q = 0; q < n; q++) {
-        float y = out[q * 5] * ip;
-        for (int k = 0; k < 4; k++) out[q * 5 + 1 + k] = (out[q * 5 + 1 + k] - y * lp_d[k]) * ip;
-        out[q * 5] = y;
-    }
-    return true;
-}
-
 // ---------------------------------------------------------------------------
-// The same sweep by a warp, for the SVI's steps (metzger_dual_raw's arithmetic
-// and results).  Of a step's ~300 instructions all but the energy, velocity
-// and radius recursion depend on the grid time alone: the lanes first form the
-// 200 grid rows and their t0 tangents, then lanes 0..3 run the recursion (lane
-// k with the tangent of parameter k), and the lanes interpolate the
-// observations.  The recursion's 200 dependent steps are what is left of the
-// chain.
+// The sweep by a warp (the SVI's steps, and lcf_svi_elbo_grad).  Of a grid
+// step's ~300 instructions all but the energy, velocity and radius recursion
+// depend on the grid time alone: the lanes first form the 200 grid rows and
+// their t0 tangents, then lanes 0..3 run the recursion (lane k with the tangent
+// of parameter k), and the lanes interpolate the observations.  The recursion's
+// 200 dependent steps are what is left of the chain.
 // ---------------------------------------------------------------------------
-// a * b with the tangent's two products rounded in a fixed order, the one the
-// compiler gives metzger_dual_raw at the place in question: the first form
-// rounds a'b before the sum, the second ab'.  (Whichever product is fused, the
-// tangent is good to an ulp; the recursion amplifies an ulp, so the two sweeps
-// have to agree.)
+// a * b with the tangent's two products rounded in a fixed order: the first
+// form rounds a'b before the sum, the second ab'.  Whichever product is fused,
+// the tangent is good to an ulp, but the recursion amplifies an ulp, so the
+// order is written down at the places that feed it: a fit keeps its bits
+// whatever the compiler would contract there.
 __device__ __forceinline__ DN<1> mul_round_first(const DN<1>& a, const DN<1>& b) {
     DN<1> r;
     r.v = a.v * b.v;
@@ -244,7 +112,7 @@ __device__ __forceinline__ DN<1> mul_round_second(const DN<1>& a, const DN<1>& b
     return r;
 }
 // Keeps a value's own rounding: the compiler must not contract the product
-// behind it into a later sum (metzger_dual_raw stores it in between).
+// behind it into a later sum.
 __device__ __forceinline__ void keep_rounded(DN<1>& a) {
     asm volatile("" : "+f"(a.v), "+f"(a.d[0]));
 }
@@ -273,8 +141,9 @@ __device__ __forceinline__ void metzger_dual_row(int i, const DN<1>& dl, float l
 }
 
 // One sample's normalised predictions and derivatives of the band to
-// out[j * 5 + {0..4}] (metzger_dual_sweep's values); pv is uniform over the
-// warp.
+// out[j * 5 + {0..4}], for observation times in ascending order; pv is uniform
+// over the warp.  All zeros where the reference returns zeros (phase_max <=
+// 0.01, or a non-positive or non-finite peak).
 template <class Times>
 __device__ __forceinline__ void metzger_dual_warp(MzWarp& W, const float* pv, float t_last, const Times& t, int n,
                                                   float* out) {

@@ -1088,12 +1088,13 @@ void launch_svi_metzger(const DeviceBatch& d, cudaStream_t s) {
 // estimate and its gradient at caller-given variational parameters and
 // standard-normal draws, through svi_sample_loglik and the prior and entropy
 // terms of svi_band — the SVI kernel's step without Adam.  One warp per
-// parameter point; `mscr` holds 5 n floats (one MetzgerKN sweep) per warp.
+// parameter point.  MetzgerKN takes its predictions and tangents from the
+// SVI's own metzger_dual_warp: `mz` the warp's tables, `mscr` 5 n floats.
 // ---------------------------------------------------------------------------
 template <int M>
 __device__ void svi_grad_point(const float4* obs, int n, float t_last, const double* init, const double* vpar,
                                const double* eps, int n_samples, double* elbo_out, double* grad_out, int* flags_out,
-                               float* mscr) {
+                               float* mscr = nullptr, MzWarp* mz = nullptr) {
     constexpr int np = n_params_of(M), se = se_idx_of(M);
     const int lane = threadIdx.x & 31, j = lane & 7;
     const bool own = j < np;
@@ -1116,10 +1117,7 @@ __device__ void svi_grad_point(const float4* obs, int n, float t_last, const dou
         float pf[MAXP];
 #pragma unroll
         for (int q = 0; q < MAXP; q++) pf[q] = q < np ? __shfl_sync(FULL, (float)th_j, q) : 0.0f;
-        if constexpr (M == METZGER) {
-            if (lane == 0) metzger_dual_sweep(pf, t_last, otimes, n, mscr);
-            __syncwarp();
-        }
+        if constexpr (M == METZGER) metzger_dual_warp(*mz, pf, t_last, otimes, n, mscr);
         double lls, dlx;
         float dl_tot;
         int floored;
@@ -1154,41 +1152,54 @@ __device__ void svi_grad_point(const float4* obs, int n, float t_last, const dou
     }
 }
 
-__global__ void __launch_bounds__(128) svi_grad_kernel(int model, const float4* obs, int n, float t_last,
-                                                       const double* init, const double* vpar, int n_points,
-                                                       const double* eps, int n_samples, double* elbo, double* grad,
-                                                       int* flags, float* scratch) {
+constexpr int SG_BLOCK = 128;
+struct SviGradArgs {
+    const float4* obs;
+    int n;
+    float t_last;
+    const double *init, *vpar;
+    int n_points;
+    const double* eps;
+    int n_samples;
+    double *elbo, *grad;
+    int* flags;
+};
+template <int M>
+__device__ __forceinline__ void svi_grad_warp(const SviGradArgs& A, int p, float* mscr = nullptr, MzWarp* mz = nullptr) {
+    constexpr int np = n_params_of(M);
+    svi_grad_point<M>(A.obs, A.n, A.t_last, A.init, A.vpar + (size_t)p * 2 * np,
+                      A.eps + (size_t)p * A.n_samples * np, A.n_samples, A.elbo + p, A.grad + (size_t)p * 2 * np,
+                      A.flags + p, mscr, mz);
+}
+__global__ void __launch_bounds__(SG_BLOCK) svi_grad_kernel(int model, SviGradArgs A) {
     const int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (p >= n_points) return;
-    const int np = n_params_of(model);
-    const double* vp = vpar + (size_t)p * 2 * np;
-    const double* ep = eps + (size_t)p * n_samples * np;
-    double* g = grad + (size_t)p * 2 * np;
-    float* ms = scratch + (size_t)p * 5 * n;
+    if (p >= A.n_points) return;
     switch (model) {
-        case BAZIN: svi_grad_point<BAZIN>(obs, n, t_last, init, vp, ep, n_samples, elbo + p, g, flags + p, ms); break;
-        case VILLAR: svi_grad_point<VILLAR>(obs, n, t_last, init, vp, ep, n_samples, elbo + p, g, flags + p, ms); break;
-        case TDE: svi_grad_point<TDE>(obs, n, t_last, init, vp, ep, n_samples, elbo + p, g, flags + p, ms); break;
-        case ARNETT: svi_grad_point<ARNETT>(obs, n, t_last, init, vp, ep, n_samples, elbo + p, g, flags + p, ms); break;
-        case MAGNETAR:
-            svi_grad_point<MAGNETAR>(obs, n, t_last, init, vp, ep, n_samples, elbo + p, g, flags + p, ms);
-            break;
-        case SHOCK: svi_grad_point<SHOCK>(obs, n, t_last, init, vp, ep, n_samples, elbo + p, g, flags + p, ms); break;
-        case AFTERGLOW:
-            svi_grad_point<AFTERGLOW>(obs, n, t_last, init, vp, ep, n_samples, elbo + p, g, flags + p, ms);
-            break;
-        default: svi_grad_point<METZGER>(obs, n, t_last, init, vp, ep, n_samples, elbo + p, g, flags + p, ms); break;
+        case BAZIN: svi_grad_warp<BAZIN>(A, p); break;
+        case VILLAR: svi_grad_warp<VILLAR>(A, p); break;
+        case TDE: svi_grad_warp<TDE>(A, p); break;
+        case ARNETT: svi_grad_warp<ARNETT>(A, p); break;
+        case MAGNETAR: svi_grad_warp<MAGNETAR>(A, p); break;
+        case SHOCK: svi_grad_warp<SHOCK>(A, p); break;
+        default: svi_grad_warp<AFTERGLOW>(A, p); break;
     }
+}
+// MetzgerKN apart, so that its tables take no shared memory of the others
+__global__ void __launch_bounds__(SG_BLOCK) svi_grad_metzger_kernel(SviGradArgs A, float* scratch) {
+    __shared__ MzWarp mz[SG_BLOCK / 32];
+    const int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (p >= A.n_points) return;
+    svi_grad_warp<METZGER>(A, p, scratch + (size_t)p * 5 * A.n, &mz[threadIdx.x >> 5]);
 }
 
 void launch_svi_grad(int model, const float4* obs, int n, float t_last, const double* init, const double* vpar,
                      int n_points, const double* eps, int n_samples, double* elbo, double* grad, int* flags,
                      float* scratch, cudaStream_t s) {
     if (n_points <= 0) return;
-    const int block = 128;
-    const int64_t threads = (int64_t)n_points * 32;
-    svi_grad_kernel<<<(int)((threads + block - 1) / block), block, 0, s>>>(model, obs, n, t_last, init, vpar, n_points,
-                                                                         eps, n_samples, elbo, grad, flags, scratch);
+    const SviGradArgs args = {obs, n, t_last, init, vpar, n_points, eps, n_samples, elbo, grad, flags};
+    const int blocks = (int)(((int64_t)n_points * 32 + SG_BLOCK - 1) / SG_BLOCK);
+    if (model == METZGER) svi_grad_metzger_kernel<<<blocks, SG_BLOCK, 0, s>>>(args, scratch);
+    else svi_grad_kernel<<<blocks, SG_BLOCK, 0, s>>>(model, args);
 }
 
 }  // namespace lcf
