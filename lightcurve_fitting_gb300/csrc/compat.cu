@@ -490,8 +490,8 @@ void launch_batch_pso_cost(const double* all_times, const double* all_flux, cons
                            const int* all_is_upper, const double* all_upper_flux, const int* source_offsets,
                            const double* positions, double* costs, int n_sources, int n_particles, int n_params,
                            int model_id, int, int) {
+    if (n_sources <= 0 || n_particles <= 0 || n_params < 1 || n_params > lcf::MAXP || model_id < 0 || model_id > 7) return;
     const int64_t rows = (int64_t)n_sources * n_particles;
-    if (rows <= 0 || n_params < 1 || n_params > lcf::MAXP || model_id < 0 || model_id > 7) return;
     if (model_id == 7) {
         pso_cost_metzger_kernel<<<(int)((rows * 32 + 255) / 256), 256>>>(all_times, all_flux, all_obs_var, all_is_upper,
                                                                          all_upper_flux, source_offsets, positions,
