@@ -68,13 +68,6 @@ void eval_draws(int m, const double* p, const double* t, double* o, int nd, int 
     eval_draws_kernel<<<(int)((total + 255) / 256), 256>>>(m, p, t, o, nd, nt, np);
 }
 
-// The reference GPU kernels' model value at one time: the analytic models as
-// the CPU path, MetzgerKN by its per-observation ODE (cuda/models_device.h:
-// 458-470).
-__device__ __forceinline__ double gpu_model_at(int m, const double* p, double t) {
-    return m == 7 ? lcf::metzger_at_obs_f64(p, t) : lcf::eval_model_f64(m, p, t);
-}
-
 // One observation's term of the reference GPU cost (cuda/models.cu:546-581):
 // (pred - y)^2 / v + ln v for a detection, -ln Phi((u - pred) / sqrt v) for
 // an upper limit, with v = obs_var + sigma_extra^2.  No 1/2, no prior, no
@@ -168,7 +161,8 @@ __global__ void __launch_bounds__(COST_BLOCK) pso_cost_kernel(const double* all_
 }
 
 // MetzgerKN: one warp per row, its lanes over the observations (each
-// observation integrates its own ODE, which dwarfs the rest).
+// observation integrates its own ODE, cuda/models_device.h:458-470, which
+// dwarfs the rest).
 __global__ void __launch_bounds__(256) pso_cost_metzger_kernel(const double* all_t, const double* all_f,
                                                                const double* all_var, const int* all_up,
                                                                const double* all_uf, const int* offs,
