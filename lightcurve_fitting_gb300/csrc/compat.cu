@@ -498,12 +498,17 @@ void launch_batch_pso_cost(const double* all_times, const double* all_flux, cons
                                       pso_cost_kernel<4>, pso_cost_kernel<5>, pso_cost_kernel<6>};
     // particles a block: up to 42 (three slots or more, in equal chunks), fewer
     // (down to 2) where that leaves the chip short of four rounds of blocks
-    // (152 SMs x 8 resident): a smaller chunk gives its particles more slots,
-    // so shorter chains of observations and a shorter tail (1,000 uneven bands
-    // x 40, Villar: 1.08 ms with one chunk, 0.78 with this rule, 1.31 for a warp a row)
+    // (eight resident on an SM at 64 registers a thread): a smaller chunk gives
+    // its particles more slots, so shorter chains of observations and a shorter
+    // tail (1,000 uneven bands x 40, Villar: 1.08 ms with one chunk, 0.78 with
+    // this rule, 1.31 for a warp a row)
+    int device = 0, sms = 1;
+    cudaGetDevice(&device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    const int64_t enough = 4 * (int64_t)sms * 8;
     int chunk = (n_particles + 41) / 42;
     chunk = (n_particles + chunk - 1) / chunk;
-    while (chunk > 2 && (int64_t)n_sources * ((n_particles + chunk - 1) / chunk) < 4 * 152 * 8) chunk = (chunk + 1) / 2;
+    while (chunk > 2 && (int64_t)n_sources * ((n_particles + chunk - 1) / chunk) < enough) chunk = (chunk + 1) / 2;
     const unsigned blocks = (unsigned)n_sources * (unsigned)((n_particles + chunk - 1) / chunk);
     kernels[model_id]<<<blocks, COST_BLOCK>>>(all_times, all_flux, all_obs_var, all_is_upper, all_upper_flux,
                                               source_offsets, positions, costs, n_particles, n_params, chunk);
