@@ -561,8 +561,12 @@ static int prepare_layout(lcf_ctx* ctx, int n_sources, int n_bands, int64_t n_ob
     ctx->lb_n_mid = n_mid;
     // Swarms run by whole blocks (pso.cu): a block costs more than eight warps
     // do, so only the few longest bands, which a launch would otherwise wait
-    // for, up to a few per SM (24 swarms a band in model selection, 3 to 8 a
-    // source in the later launches)
+    // for, up to a few swarms per SM: 24 swarms a band in model selection, 3 to
+    // 8 a source in the t0 search and MultiBazin.  The gated launch, up to 21 a
+    // band of those that Bazin does not fit, takes the later launches' limit:
+    // with model selection's it measured the same within 2 % from 30 to 300
+    // long bands (90 x 600 points 100.8 ms both, 294 x 300 58 and 60, 294 x
+    // 1,500 309 and 305)
     ctx->team_obs0 = team_length(ctx->h_boff, n_bands, 64);
     ctx->team_obs = team_length(ctx->h_boff, n_bands, 300);
     // capacity
