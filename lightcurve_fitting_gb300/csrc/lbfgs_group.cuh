@@ -30,8 +30,8 @@
 // different points of it made it slower).  The warps of a block run a round
 // in step: a block barrier before and after the evaluation, so that they
 // fetch the same code.  On small batches too: 1,000 uneven sources polish in 79 ms in step
-// and in 96 ms without the barriers.  The group's scalar state and the per-lane
-// vectors live in shared memory, leaving the registers to the evaluation.
+// and in 96 ms without the barriers.  The group's scalar state and the
+// per-lane vectors wait in shared memory, leaving the registers to the evaluation.
 //
 // Where the batch leaves warps free, a band gets a whole warp: four
 // observations then go through the term for one fetch of it, and
@@ -58,20 +58,32 @@
 
 namespace lcf {
 
-// A group's scalar state (its band, the restart reduction, the polish and
-// the line search, its work counters), in shared memory: the group's eight
-// lanes write the same values and read them back by broadcast.  Kept out of
-// the registers, it leaves them to the cost evaluation, which is bound by
-// latency and so by the warps resident per SM.
-struct LbGroupState {
-    double best_c, acc0, acc1, acc2;
+// A group's scalar state, in shared memory during the cost evaluation, which is
+// bound by latency and so by the warps resident per SM: kept out of the
+// registers there.  Each lane of the group works on a copy of its own and all
+// write the same values back, with a barrier between the last read and the
+// first write: no lane may read what another has moved on, converged or not.
+// LbScalars, the polish and its line search, is read and written every round,
+// the band and the choice of the restart only where they change.  (One source's
+// polish 6.5 ms, 1,000 sources' 86; with the scalars updated in place by all
+// lanes the same.)
+struct alignas(16) LbScalars {
     double f, prev_f, best_f;
     double dginit, dgtest, finit, width, width1, stx, fx, dgx, sty, fy, dgy, stp, stmin, stmax;
-    double t_first, t_last, inv_nd;
-    unsigned long long c_pol, c_it, c_ev, c_obs, c_fp64;
-    int64_t off;
-    int n, b, acc_mask, nc, best_r, cm, head, it, evals, fp64_evals, infoc, ls_iter;
+    int cm, head, it, evals, fp64_evals, infoc, ls_iter;
     bool brackt, stage1;
+};
+struct LbBand {
+    double t_first, t_last, inv_nd;
+    int64_t off;
+    int n, b;
+};
+struct LbRestarts {
+    double best_c, acc[3];
+    int acc_mask, nc, best_r;
+};
+struct LbCounts {
+    unsigned long long pol, it, ev, obs, fp64;
 };
 
 // Per warp, in shared memory: the curvature pairs, 1 / (y.s) and the
@@ -79,7 +91,10 @@ struct LbGroupState {
 struct LbWarpShared {
     double S[7][32], Y[7][32], rho[7][32], alpha[7][32];
     double V[7][32];  // per lane: x, g, search direction, trial point and gradient, best point, swarm point
-    LbGroupState st[4];
+    LbScalars st[4];
+    LbBand band[4];
+    LbRestarts rs[4];
+    LbCounts counts[4];  // written by the group's first lane
 };
 
 // a.b over the eight lanes of this lane's group (mask gm)
@@ -362,12 +377,8 @@ __device__ LCF_LB_QUEUE_ATTR void polish_queue(const DeviceBatch& d, LbWarpShare
     double &x = sh.V[0][lane], &g = sh.V[1][lane], &dv = sh.V[2][lane], &xo = sh.V[3][lane], &go = sh.V[4][lane],
            &bx = sh.V[5][lane], &pj = sh.V[6][lane];
     x = g = dv = xo = go = bx = pj = 0.0;
-    // the group's scalars
-    LbGroupState& st = sh.st[lane / G];
-    int& b = st.b;
-    // the restart reduction
-    double &best_c = st.best_c, &acc0 = st.acc0, &acc1 = st.acc1, &acc2 = st.acc2;
-    int &acc_mask = st.acc_mask, &nc = st.nc, &best_r = st.best_r;
+    // the group's scalars: this lane's copy
+    LbScalars st;
     // the polish
     double &f = st.f, &prev_f = st.prev_f, &best_f = st.best_f;
     int &cm = st.cm, &head = st.head, &it = st.it, &evals = st.evals, &fp64_evals = st.fp64_evals;
@@ -377,14 +388,6 @@ __device__ LCF_LB_QUEUE_ATTR void polish_queue(const DeviceBatch& d, LbWarpShare
     double &stp = st.stp, &stmin = st.stmin, &stmax = st.stmax;
     int &infoc = st.infoc, &ls_iter = st.ls_iter;
     bool &brackt = st.brackt, &stage1 = st.stage1;
-    b = 0;
-    st.n = 0;
-    st.off = 0;
-    st.t_first = st.t_last = 0.0;
-    st.inv_nd = 1.0;
-    best_c = acc0 = acc1 = acc2 = INFINITY;
-    acc_mask = nc = 0;
-    best_r = -1;
     f = 0.0;
     prev_f = best_f = INFINITY;
     cm = it = evals = fp64_evals = 0;
@@ -394,10 +397,14 @@ __device__ LCF_LB_QUEUE_ATTR void polish_queue(const DeviceBatch& d, LbWarpShare
     ls_iter = 0;
     brackt = false;
     stage1 = true;
-    st.c_pol = st.c_it = st.c_ev = st.c_obs = st.c_fp64 = 0;
+    LbBand& band = sh.band[lane / G];
+    LbRestarts& rs = sh.rs[lane / G];
+    LbCounts& counts = sh.counts[lane / G];
+    band = {0.0, 0.0, 1.0, 0, 0, 0};
+    counts = {0, 0, 0, 0, 0};
 
-    auto restarts = [&]() { return d.pso_res + (size_t)(b * 8 + MODEL) * 3; };
-    auto finish = [&](double cost) {
+    auto restarts = [&](int b) { return d.pso_res + (size_t)(b * 8 + MODEL) * 3; };
+    auto finish = [&](int b, double cost) {
         ModelFit& F = d.fits[b * 8 + MODEL];
         if (gl == 0) F.cost = cost;
         if (gl < MAXP) F.params[gl] = gl < np ? pj : NAN;
@@ -413,28 +420,22 @@ __device__ LCF_LB_QUEUE_ATTR void polish_queue(const DeviceBatch& d, LbWarpShare
             i = __shfl_sync(gm, i, g0);
             if (i >= hi) {
                 phase = LB_DONE;
-                st.n = 0;
                 break;
             }
-            b = d.polish_order[i];
+            const int b = d.polish_order[i];
             const BandStats bs = d.stats[b];
             if (!bs.valid) continue;
-            const PsoResult* R = restarts();
+            const PsoResult* R = restarts(b);
             if (R[0].iters < 0) continue;  // this model was not fitted for this band
-            best_c = INFINITY;
-            best_r = -1;
+            double best_c = INFINITY;
+            int best_r = -1;
             for (int r = 0; r < 3; r++)
                 if (R[r].iters >= 0 && R[r].cost < best_c) { best_c = R[r].cost; best_r = r; }
             pj = (best_r >= 0 && j < np) ? pso_param(R[best_r], j) : 0.0;
             if (MODEL == METZGER || best_r < 0) {  // MetzgerKN keeps its swarm result
-                finish(best_c);
+                finish(b, best_c);
                 continue;
             }
-            st.off = bs.off;
-            st.n = bs.n;
-            st.t_first = bs.t_first;
-            st.t_last = bs.t_last;
-            st.inv_nd = 1.0 / (double)max(bs.n, 1);
             lo_j = j < np ? c_lo[MODEL][j] : 0.0;
             hi_j = j < np ? c_hi[MODEL][j] : 0.0;
             const double t0_lo = fmax(bs.t_first - 30.0, c_lo[MODEL][t0i]);
@@ -444,11 +445,13 @@ __device__ LCF_LB_QUEUE_ATTR void polish_queue(const DeviceBatch& d, LbWarpShare
             // the chosen restart's cost, and the choice among restarts within
             // the estimates' error of it, are settled on accurate costs (the
             // first strict minimum, as the reference's restart loop)
-            acc_mask = 0;
+            int acc_mask = 0;
             for (int r = 0; r < 3; r++)
                 if (R[r].iters >= 0 && (r == best_r || swarm_cost_tie(R[r].cost, best_c))) acc_mask |= 1 << r;
-            nc = __popc(acc_mask);
-            acc0 = acc1 = acc2 = INFINITY;
+            __syncwarp(gm);  // the last band's state is read
+            band = {bs.t_first, bs.t_last, 1.0 / (double)max(bs.n, 1), bs.off, bs.n, b};
+            rs = {best_c, {INFINITY, INFINITY, INFINITY}, acc_mask, __popc(acc_mask), best_r};
+            __syncwarp(gm);
             evals = 0;
             fp64_evals = 0;
             it = 0;
@@ -462,17 +465,20 @@ __device__ LCF_LB_QUEUE_ATTR void polish_queue(const DeviceBatch& d, LbWarpShare
         if constexpr (MODEL == METZGER) continue;  // never polished (every group is done)
         const bool want_grad = phase == LB_START || phase == LB_LS;
         GroupBand B;
-        B.off = st.off;
-        B.n = active ? st.n : 0;
-        B.t_first = st.t_first;
-        B.t_last = st.t_last;
-        B.inv_nd = st.inv_nd;
+        B.off = band.off;
+        B.n = active ? band.n : 0;
+        B.t_first = band.t_first;
+        B.t_last = band.t_last;
+        B.inv_nd = band.inv_nd;
         B.lo_j = lo_j;
         B.hi_j = hi_j;
         double fe = 0.0, ge = 0.0;
         int used64 = 0;
+        sh.st[lane / G] = st;
         if (__any_sync(FULL, active)) used64 = group_cost_grad<MODEL, G, V>(d, B, xe, want_grad, fe, ge);
         __syncthreads();
+        st = sh.st[lane / G];
+        __syncwarp(gm);  // read by the whole group before the next round's write
         if (!active) continue;
         fp64_evals += used64;
         // the transition of this group's phase; the steps shared by several
@@ -482,27 +488,31 @@ __device__ LCF_LB_QUEUE_ATTR void polish_queue(const DeviceBatch& d, LbWarpShare
         double fnew = 0.0, end_cost = 0.0;
         switch (phase) {
             case LB_ACC: {
-                const int r = __ffs(acc_mask) - 1;
-                if (r == 0) acc0 = fe;
-                else if (r == 1) acc1 = fe;
-                else acc2 = fe;
-                acc_mask &= acc_mask - 1;
-                const PsoResult* R = restarts();
-                if (acc_mask) {
-                    xe = j < np ? pso_param(R[__ffs(acc_mask) - 1], j) : 0.0;
+                LbRestarts q = rs;
+                __syncwarp(gm);
+                const int r = __ffs(q.acc_mask) - 1;
+                if (r == 0) q.acc[0] = fe;
+                else if (r == 1) q.acc[1] = fe;
+                else q.acc[2] = fe;
+                q.acc_mask &= q.acc_mask - 1;
+                const PsoResult* R = restarts(band.b);
+                if (q.acc_mask) {
+                    rs = q;
+                    xe = j < np ? pso_param(R[__ffs(q.acc_mask) - 1], j) : 0.0;
                     break;
                 }
-                if (nc > 1) {
-                    best_r = -1;
-                    best_c = INFINITY;
-                    if (acc0 < best_c) { best_c = acc0; best_r = 0; }
-                    if (acc1 < best_c) { best_c = acc1; best_r = 1; }
-                    if (acc2 < best_c) { best_c = acc2; best_r = 2; }
-                    if (best_r < 0) best_r = 0;
-                    pj = j < np ? pso_param(R[best_r], j) : 0.0;
+                if (q.nc > 1) {
+                    q.best_r = -1;
+                    q.best_c = INFINITY;
+                    if (q.acc[0] < q.best_c) { q.best_c = q.acc[0]; q.best_r = 0; }
+                    if (q.acc[1] < q.best_c) { q.best_c = q.acc[1]; q.best_r = 1; }
+                    if (q.acc[2] < q.best_c) { q.best_c = q.acc[2]; q.best_r = 2; }
+                    if (q.best_r < 0) q.best_r = 0;
+                    pj = j < np ? pso_param(R[q.best_r], j) : 0.0;
                 } else {
-                    best_c = best_r == 0 ? acc0 : best_r == 1 ? acc1 : acc2;
+                    q.best_c = q.best_r == 0 ? q.acc[0] : q.best_r == 1 ? q.acc[1] : q.acc[2];
                 }
+                rs = q;
                 x = pj;
                 xe = x;
                 phase = LB_START;
@@ -554,7 +564,14 @@ __device__ LCF_LB_QUEUE_ATTR void polish_queue(const DeviceBatch& d, LbWarpShare
                     dgxa = dgx - dgtest;
                     dgya = dgy - dgtest;
                 }
-                infoc = lb_cstep(stx, fxa, dgxa, sty, fya, dgya, stp, fpa, dpa, brackt, stmin, stmax);
+                // (copies: a reference into st would keep it out of the registers)
+                double stxa = stx, stya = sty, stpa = stp;
+                bool bracketed = brackt;
+                infoc = lb_cstep(stxa, fxa, dgxa, stya, fya, dgya, stpa, fpa, dpa, bracketed, stmin, stmax);
+                stx = stxa;
+                sty = stya;
+                stp = stpa;
+                brackt = bracketed;
                 if (modified) {
                     fx = fxa + stx * dgtest;
                     fy = fya + sty * dgtest;
@@ -586,8 +603,8 @@ __device__ LCF_LB_QUEUE_ATTR void polish_queue(const DeviceBatch& d, LbWarpShare
                 break;
             case LB_FINAL:
                 evals++;
-                end_cost = best_c;
-                if (fe < best_c && isfinite(fe)) {
+                end_cost = rs.best_c;
+                if (fe < end_cost && isfinite(fe)) {
                     pj = xe;
                     end_cost = fe;
                 }
@@ -640,7 +657,7 @@ __device__ LCF_LB_QUEUE_ATTR void polish_queue(const DeviceBatch& d, LbWarpShare
             dv = -r;
             dginit = gdot(g, dv, gm);
             if (dginit >= 0.0) {  // not a descent direction: argmin stops with an error
-                end_cost = best_c;
+                end_cost = rs.best_c;
                 do_end = true;
             } else {
                 brackt = false;
@@ -674,16 +691,20 @@ __device__ LCF_LB_QUEUE_ATTR void polish_queue(const DeviceBatch& d, LbWarpShare
             xe = xo;
         }
         if (do_end) {
-            st.c_pol++;
-            st.c_it += (unsigned long long)it;
-            st.c_ev += (unsigned long long)evals;
-            st.c_obs += (unsigned long long)evals * (unsigned long long)st.n;
-            st.c_fp64 += (unsigned long long)fp64_evals * (unsigned long long)st.n;
-            finish(end_cost);
+            if (gl == 0) {
+                counts.pol++;
+                counts.it += (unsigned long long)it;
+                counts.ev += (unsigned long long)evals;
+                counts.obs += (unsigned long long)evals * (unsigned long long)band.n;
+                counts.fp64 += (unsigned long long)fp64_evals * (unsigned long long)band.n;
+            }
+            finish(band.b, end_cost);
         }
     }
     // the work counters, summed over the warp's groups
-    unsigned long long c_pol = st.c_pol, c_it = st.c_it, c_ev = st.c_ev, c_obs = st.c_obs, c_fp64 = st.c_fp64;
+    __syncwarp();
+    unsigned long long c_pol = counts.pol, c_it = counts.it, c_ev = counts.ev, c_obs = counts.obs, c_fp64 = counts.fp64;
+    __syncwarp();
 #pragma unroll
     for (int m = G; m < 32; m <<= 1) {
         c_pol += __shfl_xor_sync(FULL, c_pol, m);
