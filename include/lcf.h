@@ -126,8 +126,8 @@ typedef struct lcf_fit_stats {
     double ms_pso;              /* model-selection PSO launch */
     double ms_lbfgs;            /* restart reduce + L-BFGS polish + BIC select */
     double ms_t0_search;        /* SVI-mode profile t0 search (two PSO launches) */
-    double ms_uncertainty;      /* SVI or Laplace */
-    double ms_refine;           /* profile refinements + mag chi2 */
+    double ms_uncertainty;      /* SVI or Laplace of the models other than MetzgerKN */
+    double ms_refine;           /* profile refinements + mag chi2, and what MetzgerKN's own stream still takes */
     double ms_multi_bazin;      /* MultiBazin K = 2..4 launches (on their own stream when branched) */
     double particle_obs_evals;  /* device-counted particle x observation evaluations in PSO launches */
     double ode_steps;           /* device-counted MetzgerKN Euler steps in PSO launches */

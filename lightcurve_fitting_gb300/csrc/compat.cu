@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(256) pso_cost_mb_kernel(const double* all_t, c
 // parameter's two draws.  The terms, sums and their order are those of one
 // lane doing it all.  One warp a block, so that a finished source frees its
 // slot at once.  Bound by the FP64 pipe.  3,000 uneven bands, 300 steps x 4
-// samples, GB300: 367 ms, against 580 ms with every lane doing all of it.
+// samples, GB300: 449 ms, against 680 ms with every lane doing all of it.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ unsigned long long xs_next(unsigned long long& x) {
     x ^= x << 13;
