@@ -68,19 +68,18 @@ MUFU_PER_ODE_STEP = 14
 FP32_PER_EVAL = {0: 24, 1: 34, 2: 30, 3: 30, 4: 26, 5: 30, 6: 32, 7: 16, 8: 24, 9: 34, 10: 44, 11: 54}
 FP32_PER_ODE_STEP = 60
 # DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) per unit of
-# work of the two reported kernels, from ncu captures of the 1,000-source
-# uneven workload: the model-selection swarm moved 86.5 MB for 6.372e9
-# particle-observation evaluations, the polish 17.3 MB for 1.510e8
-# observation-term evaluations (its bands, its swarm results and its fits;
-# no spill traffic).  A launch's traffic is scaled from these by its own
+# work of the two reported kernels, from ncu captures: the model-selection
+# swarm of 1,000 uneven sources moved 86.5 MB for 6.372e9 particle-observation
+# evaluations, the polish of 5,000 moved 261.7 MB for 7.538e8 observation-term
+# evaluations (its bands, its swarm results, its fits and a few spills).  A launch's traffic is scaled from these by its own
 # units of work.
 DRAM_BYTES_PER_PSO_OBS_EVAL = 86.54e6 / 6.372e9
-DRAM_BYTES_PER_LB_OBS_EVAL = 17.26e6 / 1.510e8
-# The polish's pipe shares in that capture (% of peak sustained): FMA 9.5,
-# FP64 23.0, issue slots 14.8, instruction-cache hit rate 56.5 %, with 18.7
-# "no instruction" stall cycles per issued instruction (bound by fetch).
-LBFGS_NCU = {"fma_pipe_pct": 9.5, "fp64_pipe_pct": 23.0, "issue_active_pct": 14.8, "icache_hit_pct": 56.5,
-             "no_instruction_stall_per_issue": 18.7}
+DRAM_BYTES_PER_LB_OBS_EVAL = 261.7e6 / 7.538e8
+# The polish's pipe shares in that capture (% of peak sustained): FMA 18.9,
+# FP64 46.7, issue slots 27.5, instruction-cache hit rate 85.4 %, with 0.83 "no
+# instruction" stall cycles per issued instruction and 6.1 at the round's barrier.
+LBFGS_NCU = {"fma_pipe_pct": 18.9, "fp64_pipe_pct": 46.7, "issue_active_pct": 27.5, "icache_hit_pct": 85.4,
+             "no_instruction_stall_per_issue": 0.83}
 # The reference's published CPU figure for its benchmark case (100 sources x
 # 3 bands x 30 points, fit_parametric(.., false, Laplace), one thread, Skylake
 # Xeon): 113-116 sources/s (benchmarks/parametric_sources.csv:2-8).
@@ -409,8 +408,8 @@ def run_fused(args, ws, rank, local):
         "particle_obs_evals": float(sum(ev)),
     }
     # the L-BFGS polish beside it: its observation-term evaluations per second
-    # of the launch, its pipe shares from ncu (it is bound by instruction
-    # fetch, not by one arithmetic pipe), and
+    # of the launch, its pipe shares from ncu (the FP64 pipe half busy, the
+    # rest the wait for the block's slowest warp), and
     # the rate its own observation terms reach streamed at full occupancy (the
     # double-float term for the evaluations it ran, the FP64 term for the range
     # fallbacks, weighted by this launch's per-model evaluations)

@@ -28,7 +28,7 @@
 
 // Linkage of the larger functions: out of line by default, so that the
 // polish's seven model terms share one copy each instead of inlining dozens
-// (the kernel is otherwise bound by instruction fetch).
+// (the kernel would otherwise wait for instructions).
 #ifndef LCF_FF_BIG
 #define LCF_FF_BIG static __device__ __noinline__
 #endif

@@ -22,8 +22,8 @@ namespace lcf {
 
 // FP64 division and square root out of line: the IEEE-rounded results of
 // the operators themselves, one copy of their instruction sequences instead
-// of one per use.  The polish is bound by instruction fetch, and the line
-// search's many divisions dominated its code.
+// of one per use.  The polish depends on its code staying short enough to be
+// fetched, and the line search's many divisions dominated it.
 #ifdef LCF_LB_INLINE_DIV
 __device__ __forceinline__ double lb_div(double a, double b) { return a / b; }
 __device__ __forceinline__ double lb_sqrt(double x) { return sqrt(x); }

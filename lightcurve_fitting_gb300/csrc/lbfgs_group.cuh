@@ -25,12 +25,15 @@
 // warp hold bands of similar length and their observation loops end
 // together.
 //
-// The polish is bound by instruction fetch (its double-float terms and FP64
-// line search are long code; measured on GB300, more resident warps at
+// The polish's double-float terms and FP64 line search are long code, and it
+// would wait for instructions (measured on GB300, more resident warps at
 // different points of it made it slower).  The warps of a block run a round
 // in step: a block barrier before and after the evaluation, so that they
-// fetch the same code.  On small batches too: 1,000 uneven sources polish in 79 ms in step
-// and in 96 ms without the barriers.  The group's scalar state and the
+// fetch the same code: 0.6 to 0.8 stall cycles an issue instead of 18.7.  1,000
+// uneven sources polish in 79 ms in step and in 96 ms without the barriers.
+// What bounds it then is the FP64 pipe, 62 % busy at 1,000 sources and 47 % at
+// 5,000, and the barrier's wait for the block's slowest warp (4.7 and 6.1
+// cycles an issue).  The group's scalar state and the
 // per-lane vectors wait in shared memory, leaving the registers to the evaluation.
 //
 // Where the batch leaves warps free, a band gets a whole warp: four

@@ -91,9 +91,10 @@ int lbfgs_grid(int num_sms) {
 
 // A batch of fewer bands than five per warp of the grid waits for its longest
 // polishes: every band then gets a warp, and the SMs start at staggered models
-// so that the models' queues drain together.  Larger batches are bound by
-// instruction fetch: eight lanes a band below 96 observations, where the
-// state machine outweighs the observations, and all blocks on one model.
+// so that the models' queues drain together.  Larger batches are bound by the
+// work: eight lanes a band below 96 observations, where the FP64 state machine
+// outweighs the observations, and all blocks on one model, whose code they
+// share.
 // Polish ms (GB300, uneven batches of 1,000 / 2,500 / 3,500 / 6,000 / 10,000
 // sources): every band a warp 79 / 161 / 222 / 405 / 644, from 96
 // observations on 100 / 188 / 244 / 328 / 500, eight lanes below 256 for all
